@@ -53,38 +53,20 @@ DRB_D float warp_max (float v)
   return v;
 }
 
-// Hull of nd control points held in shared memory (Element::get_bounds via
-// positive_get_bounds, data_model/element.hpp:150-160).
-template <int ND>
-DRB_D void warp_hull (const float *cps, float *box6, int lane)
+// Warp minimum and maximum of a float: one redux instruction (sm_100a has
+// the f32 forms) in place of five shuffle steps.  NaN lanes are ignored, as
+// fminf and fmaxf ignore them.
+DRB_D float redux_min (float v)
 {
-  float mn[3] = { INFINITY, INFINITY, INFINITY };
-  float mx[3] = { -INFINITY, -INFINITY, -INFINITY };
-  for (int i = lane; i < ND; i += kWarp)
-  {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-      const float q = cps[3 * i + k];
-      mn[k] = fminf (mn[k], q);
-      mx[k] = fmaxf (mx[k], q);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-  {
-    mn[k] = warp_min (mn[k]);
-    mx[k] = warp_max (mx[k]);
-  }
-  if (lane == 0)
-  {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-      box6[2 * k] = mn[k];
-      box6[2 * k + 1] = mx[k];
-    }
-  }
+  float r;
+  asm volatile ("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+DRB_D float redux_max (float v)
+{
+  float r;
+  asm volatile ("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
 
 // AABB::volume, falling back to AABB::surface_area when the volume is 0
@@ -116,43 +98,120 @@ DRB_D void scale_range (float &mn, float &mx, float s)
   mx = fmaxf (mx, __fadd_rn (c, delta));
 }
 
-// One half of a binary de Casteljau split at 0.5 along `axis`, in place, for
-// `lines x 3` work items spread over the warp (split_inplace<Tensor>,
-// data_model/elem_ops.hpp:1346-1405).  left: keep [0,0.5]; else [0.5,1].
-template <int DIM, int P>
-DRB_D void split_half (float *cps, int axis, bool left, int item)
+// Key of a box's measure for the warp's argmax: ordered as the floats are,
+// so that the largest key, lowest lane first, is the box that the
+// reference's scan picks (mesh_utils.cpp:586-603: replace on >, from box 0).
+// A NaN never replaces, and a NaN in box 0 is never replaced.
+DRB_D unsigned measure_key (const float (&b)[6], int lane)
 {
-  constexpr int NL = (DIM == 3) ? (P + 1) * (P + 1) : (P + 1);
-  const int line = item / 3;
-  const int k = item - 3 * line;
-  if (line >= NL) return;
-  int stride = 1;
-  for (int d = 0; d < axis; ++d) stride *= (P + 1);
-  const int chunk_sz = stride * (P + 1);
-  const int chunk = line / stride;
-  const int e = line - chunk * stride;
-  const int base = chunk * chunk_sz + e;
-  float d[P + 1];
+  const float m = box_measure (b);
+  if (m != m) return lane == 0 ? 0xffffffffu : 0u;
+  return float_to_ordered (__fadd_rn (m, 0.f)); // -0 compares equal to +0
+}
+
+DRB_D int largest_box (unsigned key)
+{
+  const unsigned best = __reduce_max_sync (0xffffffffu, key);
+  return __ffs (__ballot_sync (0xffffffffu, key == best)) - 1;
+}
+
+// Both halves of one line of a binary split at 0.5 by a single de Casteljau
+// triangle: the first values of its rows are the [0, 0.5] half, the last
+// ones the [0.5, 1] half.  The reference runs two in-place sweeps
+// (split_inplace, data_model/elem_ops.hpp:1216-1405); each of their sums is
+// one of the triangle's, of the same two products, so the bits are equal.
+// m: the line's degree (m <= P); d: its m + 1 values, first half on return.
+template <int P> DRB_D void split_line (float (&d)[P + 1], float (&second)[P + 1], int m)
+{
 #pragma unroll
-  for (int ii = 0; ii <= P; ++ii) d[ii] = cps[3 * (base + ii * stride) + k];
-  if (left)
+  for (int a = 0; a <= P; ++a) second[a] = d[a];
+#pragma unroll
+  for (int row = 1; row <= P; ++row)
+  {
+    if (row > m) break;
+#pragma unroll
+    for (int a = 0; a + row <= P; ++a)
+      if (a + row <= m) second[a] = __fadd_rn (__fmul_rn (second[a], 0.5f), __fmul_rn (second[a + 1], 0.5f));
+    // second[0 .. m - row] is row `row`; its first value ends the first half
+    d[row] = second[0];
+  }
+}
+
+// Hulls of the two halves of a split box, from each lane's extremes of the
+// values it holds (component comp[r] in round r, no values: +-INF).
+template <int ROUNDS>
+DRB_D void half_hulls (const int (&comp)[ROUNDS], const float (&lo1)[ROUNDS], const float (&hi1)[ROUNDS],
+                       const float (&lo2)[ROUNDS], const float (&hi2)[ROUNDS], float (&b1)[6],
+                       float (&b2)[6])
+{
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+  {
+    float l1 = INFINITY, h1 = -INFINITY, l2 = INFINITY, h2 = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r)
+      if (comp[r] == k)
+      {
+        l1 = fminf (l1, lo1[r]);
+        h1 = fmaxf (h1, hi1[r]);
+        l2 = fminf (l2, lo2[r]);
+        h2 = fmaxf (h2, hi2[r]);
+      }
+    b1[2 * k] = redux_min (l1);
+    b1[2 * k + 1] = redux_max (h1);
+    b2[2 * k] = redux_min (l2);
+    b2[2 * k + 1] = redux_max (h2);
+  }
+}
+
+// Hull of ND control points in shared memory, the same in every lane
+// (Element::get_bounds via positive_get_bounds, data_model/element.hpp:150-160).
+template <int ND> DRB_D void warp_hull (const float *cps, float (&box)[6], int lane)
+{
+  float mn[3] = { INFINITY, INFINITY, INFINITY };
+  float mx[3] = { -INFINITY, -INFINITY, -INFINITY };
+  for (int i = lane; i < ND; i += kWarp)
   {
 #pragma unroll
-    for (int ff = 1; ff <= P; ++ff)
-#pragma unroll
-      for (int ii = P; ii >= ff; --ii)
-        d[ii] = __fadd_rn (__fmul_rn (d[ii - 1], 0.5f), __fmul_rn (d[ii], 0.5f));
+    for (int k = 0; k < 3; ++k)
+    {
+      const float q = cps[3 * i + k];
+      mn[k] = fminf (mn[k], q);
+      mx[k] = fmaxf (mx[k], q);
+    }
   }
-  else
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
   {
-#pragma unroll
-    for (int fb = 1; fb <= P; ++fb)
-#pragma unroll
-      for (int ii = 0; ii <= P - fb; ++ii)
-        d[ii] = __fadd_rn (__fmul_rn (d[ii], 0.5f), __fmul_rn (d[ii + 1], 0.5f));
+    box[2 * k] = redux_min (mn[k]);
+    box[2 * k + 1] = redux_max (mx[k]);
   }
+}
+
+// One finished sub-box: the scaled box, its element and reference box (R
+// floats) to slot o, and its box into the block's scene bounds.
+template <int R>
+DRB_D void write_subbox (size_t o, int el, const float (&box)[6], const float *ref,
+                         float *__restrict__ aabbs6, int *__restrict__ prim_ids,
+                         float *__restrict__ ref_out, float (&bmn)[3], float (&bmx)[3])
+{
+  const float s = (float)1.000001;
+  float bx[6];
 #pragma unroll
-  for (int ii = 0; ii <= P; ++ii) cps[3 * (base + ii * stride) + k] = d[ii];
+  for (int q = 0; q < 6; ++q) bx[q] = box[q];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) scale_range (bx[2 * k], bx[2 * k + 1], s);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) aabbs6[6 * o + q] = bx[q];
+  if (prim_ids) prim_ids[o] = el;
+#pragma unroll
+  for (int q = 0; q < R; ++q) ref_out[R * o + q] = ref[q];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+  {
+    bmn[k] = fminf (bmn[k], bx[2 * k]);
+    bmx[k] = fmaxf (bmx[k], bx[2 * k + 1]);
+  }
 }
 
 // Scene bounds (reduce, linear_bvh_builder.cpp:19-58) of the boxes a block
@@ -190,6 +249,17 @@ DRB_D void reduce_scene_bounds (float (&bmn)[3], float (&bmx)[3], float (*s_boun
   }
 }
 
+// A warp per element.  Lane b owns box b: its hull and measure key in
+// registers, its reference box as the low corner and the number of halvings
+// per axis (the reference boxes are dyadic, so low + 2^-halvings is exact).
+// Only the control points live in shared memory.  A split is then an argmax
+// over the lanes' keys (the first form scanned all measures again in every
+// lane, 528 measures an element), one de Casteljau triangle per line that
+// gives both halves, and twelve redux for the two hulls (the first form ran
+// 60 shuffles).  Box NB - 1 = 32 of a hex is the last one made and never a
+// candidate, so 32 lanes suffice.  Bound by instruction issue and the latency
+// of the split's chain.  262,144 order-2 hexes: 8.0 -> 1.87 ms; 32,768 of
+// order 3: 2.0 -> 0.47 ms.
 template <int DIM, int P>
 __global__ void __launch_bounds__ (kSubboxWarps * kWarp)
 subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, int n_elem,
@@ -199,15 +269,14 @@ subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, 
   constexpr int ND = (DIM == 3) ? (P + 1) * (P + 1) * (P + 1) : (P + 1) * (P + 1);
   constexpr int NB = SplitCount<DIM>::boxes;
   constexpr int NL = (DIM == 3) ? (P + 1) * (P + 1) : (P + 1);
-  constexpr int CPW = NB * ND * 3;     // control point floats per warp
+  constexpr int CPW = NB * ND * 3; // control point floats per warp
+  constexpr int ROUNDS = (3 * NL + kWarp - 1) / kWarp;
   extern __shared__ float smem[];
   __shared__ float s_bounds[kSubboxWarps][6];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   float *cps = smem + warp * CPW;
-  float *boxes = smem + kSubboxWarps * CPW + warp * NB * 6;
-  float *refs = smem + kSubboxWarps * (CPW + NB * 6) + warp * NB * 2 * DIM;
 
   const int el = blockIdx.x * kSubboxWarps + warp;
   float bmn[3] = { INFINITY, INFINITY, INFINITY };
@@ -222,92 +291,140 @@ subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, 
       const int k = t - 3 * i;
       cps[t] = __ldg (xyz + 3 * (size_t)__ldg (ctrl_idx + (size_t)el * ND + i) + k);
     }
-    if (lane < DIM)
+    // this lane's (line, component) items: component major, and the float
+    // offset of each item's first value for a split along each axis
+    int comp[ROUNDS], first[ROUNDS][DIM];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r)
     {
-      refs[lane] = 0.f;
-      refs[DIM + lane] = 1.f;
+      const int item = lane + r * kWarp;
+      const int line = item % NL;
+      comp[r] = item < 3 * NL ? item / NL : -1;
+      int stride = 1;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+      {
+        const int chunk = line / stride;
+        first[r][d] = 3 * (chunk * stride * (P + 1) + line - chunk * stride) + comp[r];
+        stride *= P + 1;
+      }
     }
+    float box[6], low[DIM];
+    int halvings = 0; // 8 bits per axis
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) low[d] = 0.f;
     __syncwarp ();
-    warp_hull<ND> (cps, boxes, lane);
-    __syncwarp ();
+    warp_hull<ND> (cps, box, lane);
+    unsigned key = lane == 0 ? measure_key (box, lane) : 0u;
+    float last_box[6], last_low[DIM];
+    int last_halvings = 0;
 
     for (int count = 1; count < NB; ++count)
     {
-      // largest-measure box, first one on ties (mesh_utils.cpp:586-603)
-      int max_id = 0;
-      float max_measure = box_measure (boxes);
-      for (int b = 1; b < count; ++b)
-      {
-        const float m = box_measure (boxes + 6 * b);
-        if (m > max_measure)
-        {
-          max_id = b;
-          max_measure = m;
-        }
-      }
+      // largest-measure box, first one on ties
+      const int mother_id = largest_box (key);
       // pick_binary_split: longest reference axis, first on ties
-      // (mesh_utils.cpp:482-506)
-      const float *rm = refs + max_id * 2 * DIM;
-      int axis = 0;
-      float max_len = rm[DIM] - rm[0];
+      // (mesh_utils.cpp:482-506), here the one with the fewest halvings
+      int hv = __shfl_sync (0xffffffffu, halvings, mother_id);
+      int axis = 0, fewest = hv & 255;
 #pragma unroll
       for (int d = 1; d < DIM; ++d)
       {
-        const float len = rm[DIM + d] - rm[d];
-        if (len > max_len)
+        const int h = (hv >> (8 * d)) & 255;
+        if (h < fewest)
         {
           axis = d;
-          max_len = len;
+          fewest = h;
         }
       }
-      __syncwarp ();
-      if (lane == 0)
-      {
-        // split_subref<Tensor> (data_model/ref_space.hpp:148-171)
-        float *rd = refs + count * 2 * DIM;
-        float *rmw = refs + max_id * 2 * DIM;
-        const float sp = __fadd_rn (__fmul_rn (rmw[axis], 0.5f), __fmul_rn (rmw[DIM + axis], 0.5f));
+      // split_subref<Tensor> (data_model/ref_space.hpp:148-171): the
+      // daughter starts at the mother's middle
+      float dlow[DIM];
 #pragma unroll
-        for (int q = 0; q < 2 * DIM; ++q) rd[q] = rmw[q];
-        rmw[DIM + axis] = sp;
-        rd[axis] = sp;
-      }
-      float *mother = cps + max_id * ND * 3;
-      float *dghter = cps + count * ND * 3;
-      for (int t = lane; t < ND * 3; t += kWarp) dghter[t] = mother[t];
-      __syncwarp ();
-      for (int item = lane; item < 2 * NL * 3; item += kWarp)
+      for (int d = 0; d < DIM; ++d)
       {
-        const bool is_mother = item < NL * 3;
-        split_half<DIM, P> (is_mother ? mother : dghter, axis, is_mother,
-                            is_mother ? item : item - NL * 3);
+        dlow[d] = __shfl_sync (0xffffffffu, low[d], mother_id);
+        if (d == axis) dlow[d] = __fadd_rn (dlow[d], __int_as_float ((126 - fewest) << 23));
       }
-      __syncwarp ();
-      warp_hull<ND> (mother, boxes + 6 * max_id, lane);
-      warp_hull<ND> (dghter, boxes + 6 * count, lane);
+      hv += 1 << (8 * axis);
+      float *mother = cps + mother_id * ND * 3;
+      float *dghter = cps + count * ND * 3;
+      const int step = axis == 0 ? 3 : (axis == 1 ? 3 * (P + 1) : 3 * (P + 1) * (P + 1));
+      float lo1[ROUNDS], hi1[ROUNDS], lo2[ROUNDS], hi2[ROUNDS];
+#pragma unroll
+      for (int r = 0; r < ROUNDS; ++r)
+      {
+        lo1[r] = lo2[r] = INFINITY;
+        hi1[r] = hi2[r] = -INFINITY;
+        if (comp[r] >= 0)
+        {
+          int at = first[r][0];
+#pragma unroll
+          for (int d = 1; d < DIM; ++d)
+            if (axis == d) at = first[r][d];
+          float d1[P + 1], d2[P + 1];
+#pragma unroll
+          for (int a = 0; a <= P; ++a) d1[a] = mother[at + a * step];
+          split_line<P> (d1, d2, P);
+#pragma unroll
+          for (int a = 0; a <= P; ++a)
+          {
+            mother[at + a * step] = d1[a];
+            dghter[at + a * step] = d2[a];
+            lo1[r] = fminf (lo1[r], d1[a]);
+            hi1[r] = fmaxf (hi1[r], d1[a]);
+            lo2[r] = fminf (lo2[r], d2[a]);
+            hi2[r] = fmaxf (hi2[r], d2[a]);
+          }
+        }
+      }
+      float b1[6], b2[6];
+      half_hulls<ROUNDS> (comp, lo1, hi1, lo2, hi2, b1, b2);
+      const bool is_daughter = lane == count;
+      if (lane == mother_id || is_daughter)
+      {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) box[q] = is_daughter ? b2[q] : b1[q];
+        key = measure_key (box, lane);
+        halvings = hv;
+        if (is_daughter)
+        {
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) low[d] = dlow[d];
+        }
+      }
+      if (NB > kWarp && count == NB - 1)
+      {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) last_box[q] = b2[q];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) last_low[d] = dlow[d];
+        last_halvings = hv;
+      }
       __syncwarp ();
     }
 
-    const float s = (float)1.000001;
-    for (int b = lane; b < NB; b += kWarp)
+    const size_t o = (size_t)el * NB;
+    float ref[2 * DIM];
+    if (lane < NB)
     {
-      float bx[6];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) bx[q] = boxes[6 * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) scale_range (bx[2 * k], bx[2 * k + 1], s);
-      const size_t o = (size_t)el * NB + b;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) aabbs6[6 * o + q] = bx[q];
-      prim_ids[o] = el;
-#pragma unroll
-      for (int q = 0; q < 2 * DIM; ++q) ref_out[2 * DIM * o + q] = refs[2 * DIM * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
+      for (int d = 0; d < DIM; ++d)
       {
-        bmn[k] = fminf (bmn[k], bx[2 * k]);
-        bmx[k] = fmaxf (bmx[k], bx[2 * k + 1]);
+        ref[d] = low[d];
+        ref[DIM + d] = __fadd_rn (low[d], __int_as_float ((127 - ((halvings >> (8 * d)) & 255)) << 23));
       }
+      write_subbox<2 * DIM> (o + lane, el, box, ref, aabbs6, prim_ids, ref_out, bmn, bmx);
+    }
+    if (NB > kWarp && lane == 0)
+    {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+      {
+        ref[d] = last_low[d];
+        ref[DIM + d] = __fadd_rn (last_low[d], __int_as_float ((127 - ((last_halvings >> (8 * d)) & 255)) << 23));
+      }
+      write_subbox<2 * DIM> (o + NB - 1, el, last_box, ref, aabbs6, prim_ids, ref_out, bmn, bmx);
     }
   }
   reduce_scene_bounds (bmn, bmx, s_bounds, warp, lane, bounds_ord);
@@ -333,70 +450,87 @@ subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, 
 // coincide and the boxes are bit-identical to the reference's.
 
 constexpr int kTetRefFloats = 12; // SubRef<3,Simplex>: four vertices
+constexpr int kTriRefFloats = 6;  // SubRef<2,Simplex>: three vertices
 
-// One line of a tet split: the dofs with fixed exponents g, h of the two
-// vertices off the split edge, ordered by the exponent a of the displaced
-// vertex v0 (the tradeoff vertex v1 gets m - a).  De Casteljau at 0.5 in the
-// reference's update order: for nu = m..1, a = m down to m - nu + 1,
-//   C[a] = C[a] * f + C[a - 1] * (1 - f).
-template <int P>
-DRB_D void tet_split_line (float *cps, int v0, int v1, int g, int h, int comp)
+// ---- simplex faces (triangles): 17 sub-boxes per triangle ----
+//
+// The same split with dim 2: the reference sub-triangle is three vertices
+// (u and v axis vertices, then the origin), the longest of its three edges
+// is halved, and split_inplace<2,Simplex> (elem_ops.hpp:1216-1250) runs de
+// Casteljau along it on the rows parallel to it.  Its triangle index
+// (cartesian_to_tri_idx) is the evaluators' layout, so these boxes match the
+// reference's at every order.
+
+// Lines of a simplex split: for each pair of vertices (displaced v0 <
+// tradeoff v1, in the order of the edge search) and each line (the dofs with
+// fixed exponents of the other vertices), the dof with exponent a of v0 in
+// byte a.  Line l is the same (exponents, degree) for every pair.
+template <int DIM, int P> struct SimplexLines
 {
-  const int avail = 0xf & ~(1 << v0) & ~(1 << v1);
-  const int v2 = (avail & 1) ? 0 : (avail & 2) ? 1 : (avail & 4) ? 2 : 3;
-  const int v3 = 6 - v0 - v1 - v2;
-  const int m = P - g - h;
-  int ids[P + 1];
-  float d[P + 1];
-#pragma unroll
-  for (int a = 0; a <= P; ++a)
-  {
-    if (a > m) break;
-    int b[4];
-    b[v0] = a;
-    b[v1] = m - a;
-    b[v2] = g;
-    b[v3] = h;
-    ids[a] = tet_index (b[0], b[1], b[2], P);
-    d[a] = cps[3 * ids[a] + comp];
-  }
-#pragma unroll
-  for (int nu = P; nu >= 1; --nu)
-  {
-    if (nu > m) continue;
-#pragma unroll
-    for (int a = P; a >= 1; --a)
+  static constexpr int kPairs = DIM == 3 ? 6 : 3;
+  static constexpr int kLines = DIM == 3 ? (P + 1) * (P + 2) / 2 : P + 1;
+  unsigned ids[kPairs][kLines];
+  int degree[kLines];
+};
+
+template <int DIM, int P> constexpr SimplexLines<DIM, P> simplex_lines ()
+{
+  SimplexLines<DIM, P> t{};
+  int pair = 0;
+  for (int v0 = 0; v0 < DIM; ++v0)
+    for (int v1 = v0 + 1; v1 <= DIM; ++v1, ++pair)
     {
-      if (a > m || a < m - nu + 1) continue;
-      d[a] = __fadd_rn (__fmul_rn (d[a], 0.5f), __fmul_rn (d[a - 1], 0.5f));
+      int v2 = 0;
+      while (v2 == v0 || v2 == v1) ++v2;
+      const int v3 = DIM == 3 ? 6 - v0 - v1 - v2 : 0;
+      int line = 0;
+      for (int h = 0; h <= (DIM == 3 ? P : 0); ++h)
+        for (int g = 0; g + h <= P; ++g, ++line)
+        {
+          const int m = P - g - h;
+          unsigned packed = 0;
+          for (int a = 0; a <= m; ++a)
+          {
+            int b[4] = { 0, 0, 0, 0 };
+            b[v0] = a;
+            b[v1] = m - a;
+            b[v2] = g;
+            if (DIM == 3) b[v3] = h;
+            const int id = DIM == 3 ? tet_index (b[0], b[1], b[2], P) : tri_index (b[0], b[1], P);
+            packed |= (unsigned)id << (8 * a);
+          }
+          t.ids[pair][line] = packed;
+          t.degree[line] = m;
+        }
     }
-  }
-#pragma unroll
-  for (int a = 0; a <= P; ++a)
-  {
-    if (a > m) break;
-    cps[3 * ids[a] + comp] = d[a];
-  }
+  return t;
 }
 
-template <int P>
+template <int DIM, int P> __device__ const SimplexLines<DIM, P> kSimplexLines = simplex_lines<DIM, P> ();
+
+// The tensor kernel's scheme for tets (33 sub-boxes) and triangles (17).
+// The reference sub-simplices stay in shared memory (their vertices are
+// read by every lane for the edge search); every item (line, component) has
+// a lane of its own, degree-0 lines among them, which both halves share.
+template <int DIM, int P>
 __global__ void __launch_bounds__ (kSubboxWarps * kWarp)
-tet_subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, int n_elem,
-                   float *__restrict__ aabbs6, int *__restrict__ prim_ids,
-                   float *__restrict__ ref_out, unsigned *__restrict__ bounds_ord)
+simplex_subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, int n_elem,
+                       float *__restrict__ aabbs6, int *__restrict__ prim_ids,
+                       float *__restrict__ ref_out, unsigned *__restrict__ bounds_ord)
 {
-  constexpr int ND = tet_dofs<P> ();
-  constexpr int NB = SplitCount<3>::boxes;
-  constexpr int NL = P * (P + 1) / 2; // lines per split: g + h < P
+  using Lines = SimplexLines<DIM, P>;
+  constexpr int ND = DIM == 3 ? tet_dofs<P> () : tri_dofs<P> ();
+  constexpr int NB = SplitCount<DIM>::boxes;
+  constexpr int R = DIM == 3 ? kTetRefFloats : kTriRefFloats;
   constexpr int CPW = NB * ND * 3;
+  static_assert (3 * Lines::kLines <= kWarp, "one item per lane");
   extern __shared__ float smem[];
   __shared__ float s_bounds[kSubboxWarps][6];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   float *cps = smem + warp * CPW;
-  float *boxes = smem + kSubboxWarps * CPW + warp * NB * 6;
-  float *refs = smem + kSubboxWarps * (CPW + NB * 6) + warp * NB * kTetRefFloats;
+  float *refs = smem + kSubboxWarps * CPW + warp * NB * R;
 
   const int el = blockIdx.x * kSubboxWarps + warp;
   float bmn[3] = { INFINITY, INFINITY, INFINITY };
@@ -411,285 +545,110 @@ tet_subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ x
       cps[t] = __ldg (xyz + 3 * (size_t)__ldg (ctrl_idx + (size_t)el * ND + i) + k);
     }
     // ref_universe<Simplex>: unit axis vertices, then the origin
-    if (lane < kTetRefFloats) refs[lane] = (lane < 9 && lane % 4 == 0) ? 1.f : 0.f;
+    if (lane < R) refs[lane] = (lane < DIM * DIM && lane % (DIM + 1) == 0) ? 1.f : 0.f;
+    const int line = lane % Lines::kLines;
+    const int comp[1] = { lane < 3 * Lines::kLines ? lane / Lines::kLines : -1 };
+    const int degree = kSimplexLines<DIM, P>.degree[line];
+    unsigned ids[Lines::kPairs];
+#pragma unroll
+    for (int q = 0; q < Lines::kPairs; ++q) ids[q] = kSimplexLines<DIM, P>.ids[q][line];
+    float box[6];
     __syncwarp ();
-    warp_hull<ND> (cps, boxes, lane);
-    __syncwarp ();
+    warp_hull<ND> (cps, box, lane);
+    unsigned key = lane == 0 ? measure_key (box, lane) : 0u;
+    float last_box[6];
 
     for (int count = 1; count < NB; ++count)
     {
-      int max_id = 0;
-      float max_measure = box_measure (boxes);
-      for (int b = 1; b < count; ++b)
-      {
-        const float mm = box_measure (boxes + 6 * b);
-        if (mm > max_measure)
-        {
-          max_id = b;
-          max_measure = mm;
-        }
-      }
+      const int mother_id = largest_box (key);
       // pick_binary_split<Simplex>: longest reference edge (squared length
       // summed in component order), first pair on ties
-      const float *rm = refs + max_id * kTetRefFloats;
-      int dv = 0, tv = 1;
+      float *rm = refs + mother_id * R;
+      int dv = 0, tv = 1, pair = 0, q = 0;
       float max_l2 = 0.f;
-      for (int a = 0; a < 3; ++a)
-        for (int b = a + 1; b < 4; ++b)
+#pragma unroll
+      for (int a = 0; a < DIM; ++a)
+#pragma unroll
+        for (int b = a + 1; b <= DIM; ++b, ++q)
         {
-          const float e0 = __fsub_rn (rm[3 * a], rm[3 * b]);
-          const float e1 = __fsub_rn (rm[3 * a + 1], rm[3 * b + 1]);
-          const float e2 = __fsub_rn (rm[3 * a + 2], rm[3 * b + 2]);
-          const float l2 = __fadd_rn (__fadd_rn (__fmul_rn (e0, e0), __fmul_rn (e1, e1)), __fmul_rn (e2, e2));
+          float l2 = 0.f;
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+          {
+            const float e = __fsub_rn (rm[DIM * a + d], rm[DIM * b + d]);
+            l2 = d == 0 ? __fmul_rn (e, e) : __fadd_rn (l2, __fmul_rn (e, e));
+          }
           if (l2 > max_l2)
           {
             dv = a;
             tv = b;
+            pair = q;
             max_l2 = l2;
           }
         }
       __syncwarp ();
-      if (lane == 0)
+      if (lane < R)
       {
-        float *rmw = refs + max_id * kTetRefFloats;
-        float *rd = refs + count * kTetRefFloats;
-        float sp[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          sp[k] = __fadd_rn (__fmul_rn (rmw[3 * tv + k], 0.5f), __fmul_rn (rmw[3 * dv + k], 0.5f));
-#pragma unroll
-        for (int q = 0; q < kTetRefFloats; ++q) rd[q] = rmw[q];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-          rmw[3 * dv + k] = sp[k];
-          rd[3 * tv + k] = sp[k];
-        }
+        // split_subref<Simplex> (ref_space.hpp:133-146): the mother's
+        // displaced vertex and the daughter's tradeoff vertex move to the
+        // edge's middle
+        const int v = lane / DIM, d = lane - v * DIM;
+        const float sp = __fadd_rn (__fmul_rn (rm[DIM * tv + d], 0.5f), __fmul_rn (rm[DIM * dv + d], 0.5f));
+        const float keep = rm[lane];
+        __syncwarp (R == 32 ? 0xffffffffu : (1u << R) - 1u);
+        refs[count * R + lane] = v == tv ? sp : keep;
+        if (v == dv) rm[lane] = sp;
       }
-      float *mother = cps + max_id * ND * 3;
-      float *dghter = cps + count * ND * 3;
-      for (int t = lane; t < ND * 3; t += kWarp) dghter[t] = mother[t];
-      __syncwarp ();
       // mother: split (displaced dv, tradeoff tv); daughter: the complement
-      // (displaced tv, tradeoff dv); one (line, component) per lane
-      for (int item = lane; item < 2 * NL * 3; item += kWarp)
-      {
-        const bool is_mother = item < NL * 3;
-        const int it = is_mother ? item : item - NL * 3;
-        const int line = it / 3;
-        const int comp = it - 3 * line;
-        int h = 0, g = line;
-        while (g >= P - h)
-        {
-          g -= P - h;
-          ++h;
-        }
-        if (is_mother) tet_split_line<P> (mother, dv, tv, g, h, comp);
-        else tet_split_line<P> (dghter, tv, dv, g, h, comp);
-      }
-      __syncwarp ();
-      warp_hull<ND> (mother, boxes + 6 * max_id, lane);
-      warp_hull<ND> (dghter, boxes + 6 * count, lane);
-      __syncwarp ();
-    }
-
-    const float s = (float)1.000001;
-    for (int b = lane; b < NB; b += kWarp)
-    {
-      float bx[6];
-#pragma unroll
-      for (int q = 0; q < 6; ++q) bx[q] = boxes[6 * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) scale_range (bx[2 * k], bx[2 * k + 1], s);
-      const size_t o = (size_t)el * NB + b;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) aabbs6[6 * o + q] = bx[q];
-      prim_ids[o] = el;
-#pragma unroll
-      for (int q = 0; q < kTetRefFloats; ++q) ref_out[kTetRefFloats * o + q] = refs[kTetRefFloats * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-      {
-        bmn[k] = fminf (bmn[k], bx[2 * k]);
-        bmx[k] = fmaxf (bmx[k], bx[2 * k + 1]);
-      }
-    }
-  }
-  reduce_scene_bounds (bmn, bmx, s_bounds, warp, lane, bounds_ord);
-}
-
-// ---- simplex faces (triangles): 17 sub-boxes per triangle ----
-//
-// The same split with dim 2: the reference sub-triangle is three vertices
-// (u and v axis vertices, then the origin), the longest of its three edges
-// is halved, and split_inplace<2,Simplex> (elem_ops.hpp:1216-1250) runs de
-// Casteljau along it on the rows parallel to it.  Its triangle index
-// (cartesian_to_tri_idx) is the evaluators' layout, so these boxes match the
-// reference's at every order.
-
-constexpr int kTriRefFloats = 6; // SubRef<2,Simplex>: three vertices
-
-template <int P>
-DRB_D void tri_split_line (float *cps, int v0, int v1, int g, int comp)
-{
-  const int v2 = 3 - v0 - v1;
-  const int m = P - g;
-  int ids[P + 1];
-  float d[P + 1];
-#pragma unroll
-  for (int a = 0; a <= P; ++a)
-  {
-    if (a > m) break;
-    int b[3];
-    b[v0] = a;
-    b[v1] = m - a;
-    b[v2] = g;
-    ids[a] = tri_index (b[0], b[1], P);
-    d[a] = cps[3 * ids[a] + comp];
-  }
-#pragma unroll
-  for (int nu = P; nu >= 1; --nu)
-  {
-    if (nu > m) continue;
-#pragma unroll
-    for (int a = P; a >= 1; --a)
-    {
-      if (a > m || a < m - nu + 1) continue;
-      d[a] = __fadd_rn (__fmul_rn (d[a], 0.5f), __fmul_rn (d[a - 1], 0.5f));
-    }
-  }
-#pragma unroll
-  for (int a = 0; a <= P; ++a)
-  {
-    if (a > m) break;
-    cps[3 * ids[a] + comp] = d[a];
-  }
-}
-
-template <int P>
-__global__ void __launch_bounds__ (kSubboxWarps * kWarp)
-tri_subbox_kernel (const int *__restrict__ ctrl_idx, const float *__restrict__ xyz, int n_elem,
-                   float *__restrict__ aabbs6, int *__restrict__ prim_ids,
-                   float *__restrict__ ref_out, unsigned *__restrict__ bounds_ord)
-{
-  constexpr int ND = tri_dofs<P> ();
-  constexpr int NB = SplitCount<2>::boxes;
-  constexpr int CPW = NB * ND * 3;
-  extern __shared__ float smem[];
-  __shared__ float s_bounds[kSubboxWarps][6];
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  float *cps = smem + warp * CPW;
-  float *boxes = smem + kSubboxWarps * CPW + warp * NB * 6;
-  float *refs = smem + kSubboxWarps * (CPW + NB * 6) + warp * NB * kTriRefFloats;
-
-  const int el = blockIdx.x * kSubboxWarps + warp;
-  float bmn[3] = { INFINITY, INFINITY, INFINITY };
-  float bmx[3] = { -INFINITY, -INFINITY, -INFINITY };
-
-  if (el < n_elem)
-  {
-    for (int t = lane; t < ND * 3; t += kWarp)
-    {
-      const int i = t / 3;
-      const int k = t - 3 * i;
-      cps[t] = __ldg (xyz + 3 * (size_t)__ldg (ctrl_idx + (size_t)el * ND + i) + k);
-    }
-    // ref_universe<Simplex> in 2D: (1,0), (0,1), then the origin
-    if (lane < kTriRefFloats) refs[lane] = (lane == 0 || lane == 3) ? 1.f : 0.f;
-    __syncwarp ();
-    warp_hull<ND> (cps, boxes, lane);
-    __syncwarp ();
-
-    for (int count = 1; count < NB; ++count)
-    {
-      int max_id = 0;
-      float max_measure = box_measure (boxes);
-      for (int b = 1; b < count; ++b)
-      {
-        const float mm = box_measure (boxes + 6 * b);
-        if (mm > max_measure)
-        {
-          max_id = b;
-          max_measure = mm;
-        }
-      }
-      const float *rm = refs + max_id * kTriRefFloats;
-      int dv = 0, tv = 1;
-      float max_l2 = 0.f;
-      for (int a = 0; a < 2; ++a)
-        for (int b = a + 1; b < 3; ++b)
-        {
-          const float e0 = __fsub_rn (rm[2 * a], rm[2 * b]);
-          const float e1 = __fsub_rn (rm[2 * a + 1], rm[2 * b + 1]);
-          const float l2 = __fadd_rn (__fmul_rn (e0, e0), __fmul_rn (e1, e1));
-          if (l2 > max_l2)
-          {
-            dv = a;
-            tv = b;
-            max_l2 = l2;
-          }
-        }
-      __syncwarp ();
-      if (lane == 0)
-      {
-        float *rmw = refs + max_id * kTriRefFloats;
-        float *rd = refs + count * kTriRefFloats;
-        float sp[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-          sp[k] = __fadd_rn (__fmul_rn (rmw[2 * tv + k], 0.5f), __fmul_rn (rmw[2 * dv + k], 0.5f));
-#pragma unroll
-        for (int q = 0; q < kTriRefFloats; ++q) rd[q] = rmw[q];
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-        {
-          rmw[2 * dv + k] = sp[k];
-          rd[2 * tv + k] = sp[k];
-        }
-      }
-      float *mother = cps + max_id * ND * 3;
+      float *mother = cps + mother_id * ND * 3;
       float *dghter = cps + count * ND * 3;
-      for (int t = lane; t < ND * 3; t += kWarp) dghter[t] = mother[t];
-      __syncwarp ();
-      // P lines (fixed exponent g < P of the third vertex) x 3 components
-      for (int item = lane; item < 2 * P * 3; item += kWarp)
+      float lo1[1] = { INFINITY }, hi1[1] = { -INFINITY }, lo2[1] = { INFINITY }, hi2[1] = { -INFINITY };
+      if (comp[0] >= 0)
       {
-        const bool is_mother = item < P * 3;
-        const int it = is_mother ? item : item - P * 3;
-        const int g = it / 3;
-        const int comp = it - 3 * g;
-        if (is_mother) tri_split_line<P> (mother, dv, tv, g, comp);
-        else tri_split_line<P> (dghter, tv, dv, g, comp);
+        unsigned packed = ids[0];
+#pragma unroll
+        for (int p = 1; p < Lines::kPairs; ++p)
+          if (pair == p) packed = ids[p];
+        // from the tradeoff end: the daughter's half is the second one
+        float d1[P + 1], d2[P + 1];
+#pragma unroll
+        for (int a = 0; a <= P; ++a)
+          d1[a] = a <= degree ? mother[3 * ((packed >> (8 * a)) & 255) + comp[0]] : 0.f;
+        split_line<P> (d1, d2, degree);
+#pragma unroll
+        for (int a = 0; a <= P; ++a)
+          if (a <= degree)
+          {
+            const int at = 3 * ((packed >> (8 * a)) & 255) + comp[0];
+            mother[at] = d1[a];
+            dghter[at] = d2[a];
+            lo1[0] = fminf (lo1[0], d1[a]);
+            hi1[0] = fmaxf (hi1[0], d1[a]);
+            lo2[0] = fminf (lo2[0], d2[a]);
+            hi2[0] = fmaxf (hi2[0], d2[a]);
+          }
       }
-      __syncwarp ();
-      warp_hull<ND> (mother, boxes + 6 * max_id, lane);
-      warp_hull<ND> (dghter, boxes + 6 * count, lane);
+      float b1[6], b2[6];
+      half_hulls<1> (comp, lo1, hi1, lo2, hi2, b1, b2);
+      const bool is_daughter = lane == count;
+      if (lane == mother_id || is_daughter)
+      {
+#pragma unroll
+        for (int p = 0; p < 6; ++p) box[p] = is_daughter ? b2[p] : b1[p];
+        key = measure_key (box, lane);
+      }
+      if (NB > kWarp && count == NB - 1)
+      {
+#pragma unroll
+        for (int p = 0; p < 6; ++p) last_box[p] = b2[p];
+      }
       __syncwarp ();
     }
 
-    const float s = (float)1.000001;
-    for (int b = lane; b < NB; b += kWarp)
-    {
-      float bx[6];
-#pragma unroll
-      for (int q = 0; q < 6; ++q) bx[q] = boxes[6 * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) scale_range (bx[2 * k], bx[2 * k + 1], s);
-      const size_t o = (size_t)el * NB + b;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) aabbs6[6 * o + q] = bx[q];
-      prim_ids[o] = el;
-#pragma unroll
-      for (int q = 0; q < kTriRefFloats; ++q) ref_out[kTriRefFloats * o + q] = refs[kTriRefFloats * b + q];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-      {
-        bmn[k] = fminf (bmn[k], bx[2 * k]);
-        bmx[k] = fmaxf (bmx[k], bx[2 * k + 1]);
-      }
-    }
+    const size_t o = (size_t)el * NB;
+    if (lane < NB) write_subbox<R> (o + lane, el, box, refs + lane * R, aabbs6, prim_ids, ref_out, bmn, bmx);
+    if (NB > kWarp && lane == 0)
+      write_subbox<R> (o + NB - 1, el, last_box, refs + (NB - 1) * R, aabbs6, prim_ids, ref_out, bmn, bmx);
   }
   reduce_scene_bounds (bmn, bmx, s_bounds, warp, lane, bounds_ord);
 }
@@ -924,52 +883,12 @@ __global__ void pack_kernel (const int *__restrict__ ctrl_idx, const float *__re
   packed[t] = v;
 }
 
-template <int DIM, int P> size_t subbox_smem ()
-{
-  constexpr int ND = (DIM == 3) ? (P + 1) * (P + 1) * (P + 1) : (P + 1) * (P + 1);
-  constexpr int NB = SplitCount<DIM>::boxes;
-  return sizeof (float) * kSubboxWarps * (NB * ND * 3 + NB * 6 + NB * 2 * DIM);
-}
-
-template <int P> size_t tet_subbox_smem ()
-{
-  constexpr int NB = SplitCount<3>::boxes;
-  return sizeof (float) * kSubboxWarps * (NB * tet_dofs<P> () * 3 + NB * 6 + NB * kTetRefFloats);
-}
-
-template <int P>
-int launch_tri_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_boxes,
-                       unsigned *bounds_ord, cudaStream_t s)
-{
-  constexpr int NB = SplitCount<2>::boxes;
-  const size_t smem = sizeof (float) * kSubboxWarps * (NB * tri_dofs<P> () * 3 + NB * 6 + NB * kTriRefFloats);
-  cudaFuncSetAttribute (tri_subbox_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int blocks = div_up (m->n_elem, kSubboxWarps);
-  if (blocks > 0)
-    tri_subbox_kernel<P><<<blocks, kSubboxWarps * kWarp, smem, s>>> (
-    m->ctrl_idx, m->values, m->n_elem, aabbs6, prim_ids, ref_boxes, bounds_ord);
-  return check_launch ("tri_subbox_kernel");
-}
-
-template <int P>
-int launch_tet_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_boxes,
-                       unsigned *bounds_ord, cudaStream_t s)
-{
-  const size_t smem = tet_subbox_smem<P> ();
-  cudaFuncSetAttribute (tet_subbox_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                        (int)smem);
-  const int blocks = div_up (m->n_elem, kSubboxWarps);
-  if (blocks > 0)
-    tet_subbox_kernel<P><<<blocks, kSubboxWarps * kWarp, smem, s>>> (
-    m->ctrl_idx, m->values, m->n_elem, aabbs6, prim_ids, ref_boxes, bounds_ord);
-  return check_launch ("tet_subbox_kernel");
-}
-
 template <int DIM, int P>
 int launch_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_boxes,
                    unsigned *bounds_ord, cudaStream_t s)
 {
-  const size_t smem = subbox_smem<DIM, P> ();
+  constexpr int ND = (DIM == 3) ? (P + 1) * (P + 1) * (P + 1) : (P + 1) * (P + 1);
+  constexpr size_t smem = sizeof (float) * kSubboxWarps * SplitCount<DIM>::boxes * ND * 3;
   cudaFuncSetAttribute (subbox_kernel<DIM, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                         (int)smem);
   const int blocks = div_up (m->n_elem, kSubboxWarps);
@@ -979,20 +898,36 @@ int launch_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_b
   return check_launch ("subbox_kernel");
 }
 
+template <int DIM, int P>
+int launch_simplex_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_boxes,
+                           unsigned *bounds_ord, cudaStream_t s)
+{
+  constexpr int ND = DIM == 3 ? tet_dofs<P> () : tri_dofs<P> ();
+  constexpr int R = DIM == 3 ? kTetRefFloats : kTriRefFloats;
+  constexpr size_t smem = sizeof (float) * kSubboxWarps * SplitCount<DIM>::boxes * (ND * 3 + R);
+  cudaFuncSetAttribute (simplex_subbox_kernel<DIM, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                        (int)smem);
+  const int blocks = div_up (m->n_elem, kSubboxWarps);
+  if (blocks > 0)
+    simplex_subbox_kernel<DIM, P><<<blocks, kSubboxWarps * kWarp, smem, s>>> (
+    m->ctrl_idx, m->values, m->n_elem, aabbs6, prim_ids, ref_boxes, bounds_ord);
+  return check_launch ("simplex_subbox_kernel");
+}
+
 int dispatch_subbox (const drb_mesh *m, float *aabbs6, int *prim_ids, float *ref_boxes,
                      unsigned *bounds_ord, cudaStream_t s)
 {
   if (m->shape == DRB_SHAPE_SIMPLEX && m->dim == 3)
   {
-    if (m->order == 1) return launch_tet_subbox<1> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
-    if (m->order == 2) return launch_tet_subbox<2> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
-    if (m->order == 3) return launch_tet_subbox<3> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 1) return launch_simplex_subbox<3, 1> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 2) return launch_simplex_subbox<3, 2> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 3) return launch_simplex_subbox<3, 3> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
   }
   else if (m->shape == DRB_SHAPE_SIMPLEX && m->dim == 2)
   {
-    if (m->order == 1) return launch_tri_subbox<1> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
-    if (m->order == 2) return launch_tri_subbox<2> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
-    if (m->order == 3) return launch_tri_subbox<3> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 1) return launch_simplex_subbox<2, 1> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 2) return launch_simplex_subbox<2, 2> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
+    if (m->order == 3) return launch_simplex_subbox<2, 3> (m, aabbs6, prim_ids, ref_boxes, bounds_ord, s);
   }
   else if (m->shape != DRB_SHAPE_TENSOR)
   {

@@ -1,0 +1,106 @@
+"""The BVH build's kernels against NumPy restatements at the sizes where
+they can go wrong: sub-box splits (orders, partial blocks, degenerate
+elements), the radix sort and scan (edges of tiles), the bottom-up tree
+(edges of its blocks, runs of equal codes) and the wide tree's two steps.
+Everything is compared bit for bit: the steps are defined by 32-bit
+operations in a fixed order (data_model/mesh_utils.cpp:482-677,
+linear_bvh_builder.cpp:60-397)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+F = np.float32
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float32).view(np.uint32)
+
+
+# ------------------------------------------------------------ sub-boxes --
+
+def measure(b):
+    e = [F(b[2 * k + 1] - b[2 * k]) for k in range(3)]
+    v = F(F(e[0] * e[1]) * e[2])
+    if v == 0:
+        v = F(F(F(F(2) * e[0]) * e[1]) + F(F(F(2) * e[1]) * e[2]))
+        v = F(v + F(F(F(2) * e[2]) * e[0]))
+    return v
+
+
+def hull(q):
+    out = np.empty(6, F)
+    out[0::2] = np.fmin.reduce(np.vstack([q, np.full((1, 3), np.inf, F)]))
+    out[1::2] = np.fmax.reduce(np.vstack([q, np.full((1, 3), -np.inf, F)]))
+    return out
+
+
+def scaled(b):
+    out = b.copy()
+    for k in range(3):
+        lo, hi = b[2 * k], b[2 * k + 1]
+        if lo > hi:
+            continue
+        c = F(F(0.5) * F(lo + hi))
+        d = F(F(F(1.000001) * F(0.5)) * F(hi - lo))
+        out[2 * k], out[2 * k + 1] = np.fmin(lo, F(c - d)), np.fmax(hi, F(c + d))
+    return out
+
+
+def halves(q, axis, p, dim):
+    """De Casteljau at 0.5 along a lattice axis (u fastest): both halves."""
+    a = np.moveaxis(q.reshape((p + 1,) * dim + (3,)), dim - 1 - axis, 0)
+    rows = [a]
+    for _ in range(p):
+        r = rows[-1]
+        rows.append((r[:-1] * F(0.5) + r[1:] * F(0.5)).astype(F))
+    first = np.stack([rows[k][0] for k in range(p + 1)])
+    last = np.stack([rows[p - k][k] for k in range(p + 1)])
+    back = [np.moveaxis(h, 0, dim - 1 - axis).reshape(-1, 3) for h in (first, last)]
+    return back[0], back[1]
+
+
+def split_element(q, p, dim):
+    cps, refs = [q], [np.array([0.0] * dim + [1.0] * dim, F)]
+    box = [hull(q)]
+    for _ in range(2 * (2 << dim)):
+        best, m = 0, measure(box[0])
+        for b in range(1, len(box)):
+            if measure(box[b]) > m:
+                best, m = b, measure(box[b])
+        ext = refs[best][dim:] - refs[best][:dim]
+        axis = int(np.argmax(ext))
+        mid = F(F(refs[best][axis] * F(0.5)) + F(refs[best][dim + axis] * F(0.5)))
+        a, b = halves(cps[best], axis, p, dim)
+        ra, rb = refs[best].copy(), refs[best].copy()
+        ra[dim + axis] = rb[axis] = mid
+        cps[best], refs[best], box[best] = a, ra, hull(a)
+        cps.append(b), refs.append(rb), box.append(hull(b))
+    return np.stack([scaled(b) for b in box]), np.stack(refs)
+
+
+@pytest.mark.parametrize("dim,p,n", [(3, 1, 1), (3, 1, 5), (3, 2, 3), (3, 2, 4), (3, 3, 2), (3, 3, 9),
+                                     (2, 1, 5), (2, 2, 4), (2, 3, 7)])
+def test_subboxes_match_restatement(cuda, dim, p, n):
+    import torch
+    from devil_ray_b200 import api
+    rng = np.random.default_rng(100 * dim + 10 * p + n)
+    nd = (p + 1) ** dim
+    xyz = rng.uniform(-1, 1, (n, nd, 3)).astype(F)
+    xyz[0, :, 2] = F(0.25)                     # flat: volume 0, surface area decides
+    if n > 1:
+        xyz[1] = xyz[1, :1]                    # a point: every measure ties at 0
+    if n > 3:
+        xyz[3, 0, 0] = np.nan                  # ignored by the hull
+        xyz[2, :, 1] = np.nan                  # an empty range in y
+    mesh = api.UnstructuredMesh(np.arange(n * nd, dtype=np.int32), xyz.reshape(-1, 3), p, dim=dim,
+                                device=cuda)
+    got = [t.cpu().numpy() for t in api.elem_subboxes(mesh)]
+    torch.cuda.synchronize()
+    nb = 33 if dim == 3 else 17
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = [split_element(xyz[e], p, dim) for e in range(n)]
+    assert np.array_equal(got[1], np.repeat(np.arange(n, dtype=np.int32), nb))
+    for e in range(n):
+        boxes, refs = want[e]
+        assert np.array_equal(bits(got[0][e * nb:(e + 1) * nb]), bits(boxes)), f"element {e}"
+        assert np.array_equal(bits(got[2][e * nb:(e + 1) * nb]), bits(refs)), f"element {e}"
