@@ -46,7 +46,8 @@ inline int status_from (cudaError_t e)
 void set_last_error (const char *msg);
 int check_launch (const char *what);
 
-// radix sort of (key, value) pairs on the low `bits` bits of the keys
+// radix sort of (key, value) pairs on the low `bits` bits of the keys;
+// vals_in NULL: the values are the input positions
 int radix_sort_pairs (const unsigned *keys_in, const int *vals_in, unsigned *keys_out,
                       int *vals_out, int n, int bits, cudaStream_t stream);
 // exclusive prefix sum of n int32 values (in may equal out); total -> *d_total if non-null
@@ -54,20 +55,9 @@ int exclusive_scan_i32 (const int *in, int *out, int n, int *d_total, cudaStream
 
 inline int div_up (long long a, long long b) { return (int)((a + b - 1) / b); }
 
-// Workspace of the allocation-free radix sort (sizes from radix_ws_counts
-// and scan_ws_ints; kbuf/vbuf hold n elements).
-struct RadixWorkspace
-{
-  unsigned *kbuf;
-  int *vbuf;
-  int *counts;
-  int *scan_tmp;
-};
-long long radix_ws_counts (int n);
+// Ints of scan workspace for n values (exclusive_scan_i32_ws).
 int scan_ws_ints (int n);
 int exclusive_scan_i32_ws (const int *in, int *out, int n, int *d_total, int *tmp, cudaStream_t s);
-int radix_sort_pairs_ws (const unsigned *keys_in, const int *vals_in, unsigned *keys_out,
-                         int *vals_out, int n, int bits, const RadixWorkspace &ws, cudaStream_t s);
 // Batched locate with every scratch buffer supplied by the caller.
 struct LocateWorkspace
 {
@@ -76,7 +66,7 @@ struct LocateWorkspace
   unsigned *codes_sorted;
   int *iota;
   int *order;
-  RadixWorkspace radix;
+  int *scan_tmp; // scan_ws_ints (query_cell_count ()) ints
   int *hist; // query_cell_count() cell counts of the query order
 };
 // Cells of the query order (counting sort over Morton cells).

@@ -816,7 +816,7 @@ int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pt
   const int *ord = nullptr;
   if (cfg.sort_queries)
   {
-    st = cell_order (bvh, pts, n, ws.order, ws.codes, ws.iota, ws.hist, ws.radix.scan_tmp, s);
+    st = cell_order (bvh, pts, n, ws.order, ws.codes, ws.iota, ws.hist, ws.scan_tmp, s);
     if (st) return st;
     ord = ws.order;
   }

@@ -58,7 +58,7 @@ bool open_lanes (Lane (&lane)[kLanes], int chunk, cudaEvent_t start, cudaError_t
     lane[l].ws.iota = (int *)p[5];
     lane[l].ws.order = (int *)p[6];
     lane[l].ws.hist = (int *)p[7];
-    lane[l].ws.radix.scan_tmp = (int *)p[8];
+    lane[l].ws.scan_tmp = (int *)p[8];
   }
   if (e != cudaSuccess) set_last_error (cudaGetErrorString (e));
   return e == cudaSuccess;
@@ -73,7 +73,7 @@ int close_lanes (Lane (&lane)[kLanes], cudaStream_t caller, int st)
     if (!lane[l].s) continue;
     void *bufs[9] = { lane[l].pts, lane[l].cell, lane[l].ref, lane[l].ws.head, lane[l].ws.codes,
                       lane[l].ws.iota, lane[l].ws.order, lane[l].ws.hist,
-                      lane[l].ws.radix.scan_tmp };
+                      lane[l].ws.scan_tmp };
     for (void *b : bufs)
       if (b) cudaFreeAsync (b, lane[l].s);
     if (lane[l].ready)

@@ -128,7 +128,7 @@ extern "C" int drb_locate_batched_noalloc (const drb_mesh *mesh, const drb_bvh *
   ws.iota = reinterpret_cast<int *> (base + kIotaOff);
   ws.order = reinterpret_cast<int *> (base + kOrderOff);
   ws.hist = reinterpret_cast<int *> (base + kHistOff);
-  ws.radix.scan_tmp = reinterpret_cast<int *> (base + kScanOff);
+  ws.scan_tmp = reinterpret_cast<int *> (base + kScanOff);
   if ((size_t)query_cell_count () != kCellInts || scan_ws_ints ((int)kCellInts) > (int)kScanInts)
   {
     set_last_error ("locate_batched_noalloc: scratch layout does not match the query order");

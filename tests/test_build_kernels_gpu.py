@@ -104,3 +104,37 @@ def test_subboxes_match_restatement(cuda, dim, p, n):
         boxes, refs = want[e]
         assert np.array_equal(bits(got[0][e * nb:(e + 1) * nb]), bits(boxes)), f"element {e}"
         assert np.array_equal(bits(got[2][e * nb:(e + 1) * nb]), bits(refs)), f"element {e}"
+
+
+# ------------------------------------------------------- sort and scan --
+
+@pytest.mark.parametrize("n", [1, 31, 511, 4095, 4096, 4097, 3 * 4096 + 7, 300001])
+@pytest.mark.parametrize("bits_", [1, 8, 9, 30, 32])
+def test_radix_sort_is_stable_at_tile_edges(cuda, n, bits_):
+    import torch
+    from devil_ray_b200 import api
+    rng = np.random.default_rng(n + bits_)
+    keys = rng.integers(0, 1 << bits_, n, dtype=np.uint64).astype(np.uint32)
+    if n > 600:
+        keys[100:n // 2] = keys[100]           # a long run of one digit
+    k, v = api.radix_sort_pairs(torch.as_tensor(keys.view(np.int32), device=cuda),
+                                torch.arange(n, dtype=torch.int32, device=cuda), bits_)
+    order = np.argsort(keys, kind="stable")
+    assert np.array_equal(k.cpu().numpy().view(np.uint32), keys[order])
+    assert np.array_equal(v.cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 9 * 4096 + 1])
+def test_compaction_at_scan_tile_edges(cuda, n):
+    """cull_rays compacts by the exclusive scan: rays that miss a box."""
+    import torch
+    from devil_ray_b200 import render
+    rng = np.random.default_rng(n)
+    hit = rng.random(n) < 0.6
+    rays = np.zeros((n, 9), F)
+    rays[:, 2] = 1.0                            # along z
+    rays[:, 4] = np.where(hit, 0.5, 3.0)
+    rays[:, 5], rays[:, 6], rays[:, 7] = 0.5, -2.0, np.inf
+    rays[:, 8] = np.arange(n, dtype=np.int32).view(F)
+    out = render.cull_rays(torch.as_tensor(rays, device=cuda), [0, 1, 0, 1, 0, 1])
+    assert np.array_equal(out.cpu().numpy()[:, 8].view(np.int32), np.flatnonzero(hit))
