@@ -7,10 +7,8 @@
 //                   AABBs, x1.000001 scale, block-reduced scene bounds
 //   morton_kernel   30-bit codes of the scaled-box centroids
 //   radix sort      stable 4-pass LSD sort of (code, sub-box id)  (sort.cu)
-//   gather_kernel   sorted AABBs, leaf element ids
-//   karras_kernel   Karras 2012 radix tree, index tie-break
-//   refit_kernel    bottom-up AABB union with arrival counters
-//   emit_kernel     4 x float4 node records
+//   tree_kernel     Karras 2012 radix tree with index tie-break, AABB union
+//                   and 4 x float4 node records in one bottom-up pass
 //
 // Bit-exactness: the sub-box, scale, measure and Morton arithmetic use
 // explicitly rounded intrinsics (__fadd_rn/__fmul_rn/__fsub_rn) in the same
@@ -676,8 +674,7 @@ DRB_D unsigned expand_bits32 (unsigned x)
 }
 
 __global__ void morton_kernel (const float *__restrict__ aabbs6, int n,
-                               const float *__restrict__ bounds6, unsigned *__restrict__ codes,
-                               int *__restrict__ iota)
+                               const float *__restrict__ bounds6, unsigned *__restrict__ codes)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -702,160 +699,198 @@ __global__ void morton_kernel (const float *__restrict__ aabbs6, int n,
     e[k] = expand_bits32 ((unsigned)x);
   }
   codes[i] = (e[2] << 2) | (e[1] << 1) | e[0];
-  if (iota) iota[i] = i;
 }
 
-// reorder (linear_bvh_builder.cpp:99-118) of AABBs and primitive ids
-__global__ void gather_leaves_kernel (const int *__restrict__ perm, int n,
-                                      const float *__restrict__ aabbs6,
-                                      const int *__restrict__ prim_ids,
-                                      float *__restrict__ leaf_aabbs6, int *__restrict__ leaf_nodes)
+// ---- tree: Karras topology, refit and node records in one bottom-up pass --
+//
+// The reference builds the Karras 2012 radix tree top-down per node
+// (linear_bvh_builder.cpp:149-251), then refits (:253-317) and emits
+// (:319-397).  The same tree forms bottom-up (Apetrei 2014): the node over
+// the sorted leaves [l, r] joins the neighbour across its closer end, where
+// closeness is the reference's delta (common prefix of the 30-bit codes, the
+// index breaking ties), which is a strict order along any node's ends.  Of
+// the two children the second to arrive builds the parent: it has the whole
+// range, both boxes and both child codes, so the final 64-byte record is
+// written at once, and the topology arrays, the sorted box copy and two of
+// the three passes over them are not needed.  A node's index is Karras': r
+// for a left child, l for a right child, 0 for the root.  Nothing waits: the
+// first arrival leaves its box and ends.
+//
+// A block takes kTreeBlock consecutive leaves.  Joins whose result lies
+// inside the block (known beforehand from prefix and suffix minima of the
+// deltas: the result ends where the delta drops below the join's) go through
+// shared memory; only the nodes that cross a block border, a few dozen per
+// block, use global memory and its atomics.
+// 8.65M leaves: 0.67 ms, against 1.41 ms for the four kernels it replaces
+// (gather, top-down Karras, refit with global atomics, emit).  Bound by the
+// scattered 64-byte records and the box gather.
+constexpr int kTreeBlock = 256;
+
+// delta of the sorted leaves j and j + 1 (linear_bvh_builder.cpp:149-167)
+DRB_D int adjacent_delta (const unsigned *__restrict__ codes, int j, int n)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int src = perm[i];
+  if (j < 0 || j >= n - 1) return -1;
+  const unsigned x = __ldg (codes + j) ^ __ldg (codes + j + 1);
+  return x ? __clz (x) : 32 + __clz ((unsigned)j ^ (unsigned)(j + 1));
+}
+
+// Exchange with release and acquire at device scope: what a thread wrote
+// before its exchange is visible to the one that gets its value.
+DRB_D int exchange_acq_rel (int *p, int v)
+{
+  int old;
+  asm volatile ("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
+// Node record (bvh.hpp:16-37): left box, right box, child codes (4 x node
+// for an inner child, -(leaf + 1) for a leaf).  Boxes are x0 x1 y0 y1 z0 z1.
+DRB_D void write_record (float4 *__restrict__ nodes, int id, const float (&lb)[6], const float (&rb)[6],
+                         int lcode, int rcode)
+{
+  float4 *o = nodes + 4 * (size_t)id;
+  o[0] = make_float4 (lb[0], lb[2], lb[4], lb[1]);
+  o[1] = make_float4 (lb[3], lb[5], rb[0], rb[2]);
+  o[2] = make_float4 (rb[4], rb[1], rb[3], rb[5]);
+  o[3] = make_float4 (__int_as_float (lcode), __int_as_float (rcode), 0.f, 0.f);
+}
+
+// inner_box: 8 floats per inner node (32-byte sectors), met: n - 1 ints of -1.
+__global__ void __launch_bounds__ (kTreeBlock)
+tree_kernel (const unsigned *__restrict__ codes, const int *__restrict__ perm,
+             const float *__restrict__ aabbs6, int n, int boxes_per_elem, int *__restrict__ leaf_nodes,
+             float *inner_box, int *met, float4 *__restrict__ nodes)
+{
+  __shared__ int s_delta[kTreeBlock + 1];  // of leaf pairs (b0 - 1 + q, b0 + q)
+  __shared__ float s_leaf[kTreeBlock][7];  // odd stride: no bank conflicts
+  __shared__ float s_inner[kTreeBlock][7]; // by node index - b0
+  __shared__ int s_met[kTreeBlock];
+  __shared__ bool s_inside[kTreeBlock];    // join at b0 + q stays in the block
+  __shared__ int s_warp_min[2][kTreeBlock / kWarp];
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  const int b0 = blockIdx.x * kTreeBlock;
+  const int b1 = min (b0 + kTreeBlock, n);
+  const int i = b0 + tid;
+  constexpr int kFar = 1 << 20;
+
+  float box[6];
+  const int here = i < n ? adjacent_delta (codes, i, n) : kFar;
+  if (tid == 0) s_delta[0] = adjacent_delta (codes, b0 - 1, n);
+  s_delta[tid + 1] = here;
+  s_met[tid] = -1;
+  if (i < n)
+  {
+    const int src = perm[i];
+    leaf_nodes[i] = src / boxes_per_elem;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) leaf_aabbs6[6 * (size_t)i + q] = aabbs6[6 * (size_t)src + q];
-  leaf_nodes[i] = prim_ids[src];
-}
+    for (int q = 0; q < 6; ++q)
+    {
+      box[q] = __ldg (aabbs6 + 6 * (size_t)src + q);
+      s_leaf[tid][q] = box[q];
+    }
+  }
+  // minima of the deltas before and after each join
+  int before = here, after = here;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+  {
+    const int u = __shfl_up_sync (0xffffffffu, before, o);
+    const int d = __shfl_down_sync (0xffffffffu, after, o);
+    if (lane >= o) before = min (before, u);
+    if (lane + o < 32) after = min (after, d);
+  }
+  if (lane == 31) s_warp_min[0][warp] = before;
+  if (lane == 0) s_warp_min[1][warp] = after;
+  before = __shfl_up_sync (0xffffffffu, before, 1);
+  after = __shfl_down_sync (0xffffffffu, after, 1);
+  if (lane == 0) before = kFar;
+  if (lane == 31) after = kFar;
+  __syncthreads ();
+  before = min (before, s_delta[0]);
+  for (int w = 0; w < warp; ++w) before = min (before, s_warp_min[0][w]);
+  for (int w = warp + 1; w < kTreeBlock / kWarp; ++w) after = min (after, s_warp_min[1][w]);
+  s_inside[tid] = i < b1 - 1 && before < here && after < here;
+  __syncthreads ();
+  if (i >= n) return;
 
-// delta / build_tree (linear_bvh_builder.cpp:149-251), Karras 2012.
-DRB_D int karras_delta (int a, int b, int inner_size, const unsigned *__restrict__ codes)
-{
-  const bool out = (b < 0 || b > inner_size);
-  const int bb = out ? 0 : b;
-  const unsigned ac = codes[a];
-  const unsigned bc = codes[bb];
-  unsigned exor = ac ^ bc;
-  const bool tie = (exor == 0);
-  exor = tie ? ((unsigned)a ^ (unsigned)bb) : exor;
-  int count = __clz (exor);
-  if (tie) count += 32;
-  return out ? -1 : count;
-}
-
-__global__ void karras_kernel (const unsigned *__restrict__ codes, int inner_size,
-                               int *__restrict__ lchild, int *__restrict__ rchild,
-                               int *__restrict__ parent)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= inner_size) return;
-  const int d = (0 > (karras_delta (i, i + 1, inner_size, codes) -
-                      karras_delta (i, i - 1, inner_size, codes))) ? -1 : 1;
-  const int min_delta = karras_delta (i, i - d, inner_size, codes);
-  int lmax = 2;
-  while (karras_delta (i, i + lmax * d, inner_size, codes) > min_delta) lmax *= 2;
-  int l = 0;
-  for (int t = lmax / 2; t >= 1; t /= 2)
-    if (karras_delta (i, i + (l + t) * d, inner_size, codes) > min_delta) l += t;
-  const int j = i + l * d;
-  const int delta_node = karras_delta (i, j, inner_size, codes);
-  int s = 0;
-  float div_factor = 2.f;
-  for (int t = (int)ceilf (__fdiv_rn ((float)l, div_factor));;
-       div_factor *= 2.f, t = (int)ceilf (__fdiv_rn ((float)l, div_factor)))
+  int l = i, r = i, code = -(i + 1);
+  int dl = s_delta[tid], dr = here;
+  while (true)
   {
-    if (karras_delta (i, i + (s + t) * d, inner_size, codes) > delta_node) s += t;
-    if (t == 1) break;
-  }
-  const int split = i + s * d + min (d, 0);
-  if (min (i, j) == split)
-  {
-    parent[split + inner_size] = i;
-    lchild[i] = split + inner_size;
-  }
-  else
-  {
-    parent[split] = i;
-    lchild[i] = split;
-  }
-  if (max (i, j) == split + 1)
-  {
-    parent[split + inner_size + 1] = i;
-    rchild[i] = split + inner_size + 1;
-  }
-  else
-  {
-    parent[split + 1] = i;
-    rchild[i] = split + 1;
-  }
-  if (i == 0) parent[0] = -1;
-}
-
-// propagate_aabbs (linear_bvh_builder.cpp:253-317): the second thread to
-// reach a node unions its children.  The fence orders a child's box store
-// before the counter increment that releases the parent.
-__global__ void refit_kernel (const int *__restrict__ lchild, const int *__restrict__ rchild,
-                              const int *__restrict__ parent, const float *__restrict__ leaf6,
-                              float *inner6, int *counters, int inner_size, int leaf_size)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= leaf_size) return;
-  int node = parent[inner_size + i];
-  while (node != -1)
-  {
-    __threadfence ();
-    const int old = atomicAdd (counters + node, 1);
-    if (old == 0) return;
-    __threadfence ();
-    const int lc = lchild[node];
-    const int rc = rchild[node];
-    float box[6];
-    const float *lb = (lc >= inner_size) ? leaf6 + 6 * (size_t)(lc - inner_size) : inner6 + 6 * (size_t)lc;
-    const float *rb = (rc >= inner_size) ? leaf6 + 6 * (size_t)(rc - inner_size) : inner6 + 6 * (size_t)rc;
+    if (l == 0 && r == n - 1) return; // the root is written
+    const bool left = dr > dl; // a left child: the parent joins at r
+    const int p = left ? r : l - 1;
+    const bool inside = p >= b0 && p < b1 - 1 && s_inside[p - b0];
+    const int id = left ? r : l; // this node's index, if it is an inner one
+    int other;
+    if (inside)
+    {
+      if (l != r)
+      {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) s_inner[id - b0][q] = box[q];
+      }
+      __threadfence_block ();
+      other = atomicExch (&s_met[p - b0], left ? l : r);
+      if (other < 0) return;
+      __threadfence_block ();
+    }
+    else
+    {
+      if (l != r)
+      {
+        float4 *o = reinterpret_cast<float4 *> (inner_box + 8 * (size_t)id);
+        __stcg (o, make_float4 (box[0], box[1], box[2], box[3]));
+        __stcg (o + 1, make_float4 (box[4], box[5], 0.f, 0.f));
+      }
+      other = exchange_acq_rel (met + p, left ? l : r);
+      if (other < 0) return;
+    }
+    // the sibling: [p + 1, other] of a left child, [other, p] of a right one
+    const int sib_id = left ? p + 1 : p;
+    const bool sib_leaf = other == sib_id;
+    float sib[6];
+    if (inside)
+    {
+      const volatile float *sb = sib_leaf ? s_leaf[sib_id - b0] : s_inner[sib_id - b0];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) sib[q] = sb[q];
+    }
+    else if (sib_leaf)
+    {
+      const size_t src = __ldg (perm + sib_id);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) sib[q] = __ldg (aabbs6 + 6 * src + q);
+    }
+    else
+    {
+      const float4 *o = reinterpret_cast<const float4 *> (inner_box + 8 * (size_t)sib_id);
+      const float4 a = __ldcg (o), b = __ldcg (o + 1);
+      sib[0] = a.x, sib[1] = a.y, sib[2] = a.z, sib[3] = a.w, sib[4] = b.x, sib[5] = b.y;
+    }
+    const int sib_code = sib_leaf ? -(sib_id + 1) : 4 * sib_id;
+    if (left)
+    {
+      r = other;
+      dr = inside ? s_delta[r - b0 + 1] : adjacent_delta (codes, r, n);
+    }
+    else
+    {
+      l = other;
+      dl = inside ? s_delta[l - b0] : adjacent_delta (codes, l - 1, n);
+    }
+    const int parent = (l == 0 && r == n - 1) ? 0 : (dr > dl ? r : l);
+    if (left) write_record (nodes, parent, box, sib, code, sib_code);
+    else write_record (nodes, parent, sib, box, sib_code, code);
+    code = 4 * parent;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
     {
-      const float l0 = __ldcg (lb + 2 * k), l1 = __ldcg (lb + 2 * k + 1);
-      const float r0 = __ldcg (rb + 2 * k), r1 = __ldcg (rb + 2 * k + 1);
-      box[2 * k] = fminf (l0, r0);
-      box[2 * k + 1] = fmaxf (l1, r1);
+      box[2 * k] = fminf (box[2 * k], sib[2 * k]);
+      box[2 * k + 1] = fmaxf (box[2 * k + 1], sib[2 * k + 1]);
     }
-#pragma unroll
-    for (int q = 0; q < 6; ++q) __stcg (inner6 + 6 * (size_t)node + q, box[q]);
-    node = parent[node];
   }
-}
-
-// emit (linear_bvh_builder.cpp:319-397)
-__global__ void emit_kernel (const int *__restrict__ lchild, const int *__restrict__ rchild,
-                             const float *__restrict__ leaf6, const float *__restrict__ inner6,
-                             float4 *__restrict__ nodes, int inner_size)
-{
-  const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= inner_size) return;
-  int lc = lchild[node];
-  int rc = rchild[node];
-  const float *lb, *rb;
-  if (lc >= inner_size)
-  {
-    lb = leaf6 + 6 * (size_t)(lc - inner_size);
-    lc = -(lc - inner_size + 1);
-  }
-  else
-  {
-    lb = inner6 + 6 * (size_t)lc;
-    lc *= 4;
-  }
-  if (rc >= inner_size)
-  {
-    rb = leaf6 + 6 * (size_t)(rc - inner_size);
-    rc = -(rc - inner_size + 1);
-  }
-  else
-  {
-    rb = inner6 + 6 * (size_t)rc;
-    rc *= 4;
-  }
-  float4 v1 = make_float4 (lb[0], lb[2], lb[4], lb[1]);
-  float4 v2 = make_float4 (lb[3], lb[5], rb[0], rb[2]);
-  float4 v3 = make_float4 (rb[4], rb[1], rb[3], rb[5]);
-  float4 v4 = make_float4 (__int_as_float (lc), __int_as_float (rc), 0.f, 0.f);
-  float4 *o = nodes + 4 * (size_t)node;
-  o[0] = v1;
-  o[1] = v2;
-  o[2] = v3;
-  o[3] = v4;
 }
 
 template <int NC>
@@ -1079,7 +1114,7 @@ extern "C" int drb_morton_codes (const float *aabbs6, int n, const float *bounds
     return DRB_ERR_INVALID_ARG;
   }
   if (n == 0) return DRB_OK;
-  morton_kernel<<<div_up (n, 256), 256, 0, (cudaStream_t)stream>>> (aabbs6, n, bounds6, codes, nullptr);
+  morton_kernel<<<div_up (n, 256), 256, 0, (cudaStream_t)stream>>> (aabbs6, n, bounds6, codes);
   return check_launch ("morton_kernel");
 }
 
@@ -1134,39 +1169,29 @@ extern "C" int drb_lbvh_build (const drb_mesh *mesh, drb_bvh *bvh, unsigned *sor
   Scratch scr (s);
   const int n = n_leaf;
   float *aabbs = scr.alloc<float> ((size_t)6 * n);
-  int *prim = scr.alloc<int> (n);
   unsigned *codes = scr.alloc<unsigned> (n);
   unsigned *codes_sorted = sorted_codes ? sorted_codes : scr.alloc<unsigned> (n);
-  int *iota = scr.alloc<int> (n);
-  float *leaf6 = scr.alloc<float> ((size_t)6 * n);
-  int *lch = scr.alloc<int> (n_inner);
-  int *rch = scr.alloc<int> (n_inner);
-  int *par = scr.alloc<int> ((size_t)n + n_inner);
-  float *inner6 = scr.alloc<float> ((size_t)6 * n_inner);
-  int *counters = scr.alloc<int> (n_inner);
+  float *inner_box = scr.alloc<float> ((size_t)8 * n_inner);
+  int *met = scr.alloc<int> (n_inner);
   unsigned *bord = scr.alloc<unsigned> (8);
   float *bounds6 = scr.alloc<float> (8);
   if (scr.err != cudaSuccess) return status_from (scr.err);
 
   bounds_init_kernel<<<1, 32, 0, s>>> (bord);
   if ((st = check_launch ("bounds_init_kernel"))) return st;
-  st = dispatch_subbox (mesh, aabbs, prim, bvh->ref_boxes, bord, s);
+  st = dispatch_subbox (mesh, aabbs, nullptr, bvh->ref_boxes, bord, s);
   if (st) return st;
   bounds_finish_kernel<<<1, 32, 0, s>>> (bord, bounds6);
   if ((st = check_launch ("bounds_finish_kernel"))) return st;
-  morton_kernel<<<div_up (n, 256), 256, 0, s>>> (aabbs, n, bounds6, codes, iota);
+  morton_kernel<<<div_up (n, 256), 256, 0, s>>> (aabbs, n, bounds6, codes);
   if ((st = check_launch ("morton_kernel"))) return st;
-  st = radix_sort_pairs (codes, iota, codes_sorted, bvh->aabb_ids, n, 30, s);
+  st = radix_sort_pairs (codes, nullptr, codes_sorted, bvh->aabb_ids, n, 30, s);
   if (st) return st;
-  gather_leaves_kernel<<<div_up (n, 256), 256, 0, s>>> (bvh->aabb_ids, n, aabbs, prim, leaf6, bvh->leaf_nodes);
-  if ((st = check_launch ("gather_leaves_kernel"))) return st;
-  karras_kernel<<<div_up (n_inner, 256), 256, 0, s>>> (codes_sorted, n_inner, lch, rch, par);
-  if ((st = check_launch ("karras_kernel"))) return st;
-  cudaMemsetAsync (counters, 0, sizeof (int) * (size_t)n_inner, s);
-  refit_kernel<<<div_up (n, 256), 256, 0, s>>> (lch, rch, par, leaf6, inner6, counters, n_inner, n);
-  if ((st = check_launch ("refit_kernel"))) return st;
-  emit_kernel<<<div_up (n_inner, 256), 256, 0, s>>> (lch, rch, leaf6, inner6, (float4 *)bvh->inner_nodes, n_inner);
-  if ((st = check_launch ("emit_kernel"))) return st;
+  cudaMemsetAsync (met, 0xff, sizeof (int) * (size_t)n_inner, s);
+  tree_kernel<<<div_up (n, kTreeBlock), kTreeBlock, 0, s>>> (codes_sorted, bvh->aabb_ids, aabbs, n,
+                                                             n / mesh->n_elem, bvh->leaf_nodes, inner_box,
+                                                             met, (float4 *)bvh->inner_nodes);
+  if ((st = check_launch ("tree_kernel"))) return st;
   float hb[8];
   cudaError_t e = cudaMemcpyAsync (hb, bounds6, sizeof (float) * 6, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize (s);

@@ -138,3 +138,75 @@ def test_compaction_at_scan_tile_edges(cuda, n):
     rays[:, 8] = np.arange(n, dtype=np.int32).view(F)
     out = render.cull_rays(torch.as_tensor(rays, device=cuda), [0, 1, 0, 1, 0, 1])
     assert np.array_equal(out.cpu().numpy()[:, 8].view(np.int32), np.flatnonzero(hit))
+
+
+# ---------------------------------------------------------------- trees --
+
+def delta(codes):
+    """Common prefix of neighbouring codes, the index breaking ties
+    (linear_bvh_builder.cpp:149-167)."""
+    out = np.empty(len(codes) - 1, int)
+    for j in range(len(codes) - 1):
+        x = int(codes[j]) ^ int(codes[j + 1])
+        out[j] = 32 - x.bit_length() if x else 64 - (j ^ (j + 1)).bit_length()
+    return out
+
+
+def radix_tree(codes, boxes):
+    """Node records of the Karras tree, by recursion over the split with the
+    shortest prefix; boxes: sorted leaf boxes x0 x1 y0 y1 z0 z1."""
+    n = len(codes)
+    d = delta(codes)
+    rec = np.zeros((n - 1, 16), F)
+    kids = rec.view(np.int32)
+
+    def visit(l, r, left):
+        """(child code, box) of the node over [l, r], a left child or not."""
+        if l == r:
+            return -(l + 1), boxes[l]
+        me = 0 if (l, r) == (0, n - 1) else (r if left else l)
+        p = l + int(np.argmin(d[l:r]))
+        (cl, bl), (cr, br) = visit(l, p, True), visit(p + 1, r, False)
+        rec[me, :12] = np.concatenate([bl[0::2], bl[1::2], br[0::2], br[1::2]])
+        kids[me, 12], kids[me, 13] = cl, cr
+        u = np.empty(6, F)
+        u[0::2], u[1::2] = np.fmin(bl[0::2], br[0::2]), np.fmax(bl[1::2], br[1::2])
+        return 4 * me, u
+
+    visit(0, n - 1, False)
+    return rec
+
+
+def _tree_mesh(kind, n_elem, cuda):
+    from devil_ray_b200 import api
+    rng = np.random.default_rng(n_elem)
+    if kind == "scattered":
+        xyz = rng.uniform(0, 1, (n_elem, 1, 3)) + 0.1 * rng.uniform(0, 1, (n_elem, 8, 3))
+        idx = np.arange(8 * n_elem)
+    elif kind == "repeated":  # one element n times: every code occurs n times
+        xyz, idx = rng.uniform(0, 1, (1, 8, 3)), np.tile(np.arange(8), n_elem)
+    else:                     # points in one place: all codes equal
+        xyz, idx = np.full((1, 8, 3), 0.5), np.tile(np.arange(8), n_elem)
+    return api.UnstructuredMesh(idx.astype(np.int32), xyz.reshape(-1, 3).astype(F), 1, device=cuda)
+
+
+# 33 leaves an element; the tree's blocks hold 256 leaves
+@pytest.mark.parametrize("kind,n_elem", [("scattered", 1), ("scattered", 7), ("scattered", 8),
+                                         ("scattered", 31), ("scattered", 256), ("repeated", 8),
+                                         ("repeated", 70), ("point", 1), ("point", 40)])
+def test_bottom_up_tree_matches_top_down(cuda, kind, n_elem):
+    import sys
+    import torch
+    from devil_ray_b200 import api
+    mesh = _tree_mesh(kind, n_elem, cuda)
+    b = mesh.build_bvh(keep_codes=True)
+    aabbs, _, refs, bounds = api.elem_subboxes(mesh)
+    codes = api.morton_codes(aabbs, bounds).cpu().numpy().view(np.uint32)
+    torch.cuda.synchronize()
+    order = np.argsort(codes, kind="stable")
+    assert np.array_equal(b.sorted_codes.cpu().numpy().view(np.uint32), codes[order])
+    assert np.array_equal(b.aabb_ids.cpu().numpy(), order)
+    assert np.array_equal(b.leaf_nodes.cpu().numpy(), order // 33)
+    sys.setrecursionlimit(20000)
+    want = radix_tree(codes[order], aabbs.cpu().numpy()[order])
+    assert np.array_equal(bits(b.inner_nodes.cpu().numpy()), bits(want))
