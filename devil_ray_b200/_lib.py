@@ -177,6 +177,9 @@ _SIGS = {
                                  C.c_void_p, C.c_void_p]),
     "drb_mesh_face_neighbors": (C.c_int, [C.POINTER(DrbMesh), C.c_void_p, C.c_void_p]),
     "drb_bvh_widen": (C.c_int, [C.POINTER(DrbBvh), C.c_void_p, C.c_int, C.c_void_p]),
+    "drb_bvh_widen_plan": (C.c_int, [C.POINTER(DrbBvh), C.c_void_p, C.c_void_p]),
+    "drb_bvh_widen_emit": (C.c_int, [C.POINTER(DrbBvh), C.c_void_p, C.c_void_p, C.c_int,
+                                     C.c_void_p]),
     "drb_locate": (C.c_int, [C.POINTER(DrbMesh), C.POINTER(DrbBvh), C.c_void_p, C.c_int,
                              C.POINTER(DrbNewtonOpts), C.c_void_p, C.c_void_p, DrbQueryStats,
                              C.c_void_p]),

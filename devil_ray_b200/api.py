@@ -135,11 +135,15 @@ class BVH:
         """Build the 4-wide traversal tree of this BVH (same candidates in
         the same order; one 128-byte node per two binary levels)."""
         d = self.desc()
-        L.check(L.lib().drb_bvh_widen(C.byref(d), None, 0, _stream(stream)), "drb_bvh_widen")
-        self.wide_nodes = torch.empty((max(d.n_wide, 1), 32), dtype=torch.float32,
-                                      device=self.inner_nodes.device)
-        L.check(L.lib().drb_bvh_widen(C.byref(d), _ptr(self.wide_nodes), d.n_wide,
-                                      _stream(stream)), "drb_bvh_widen")
+        dev = self.inner_nodes.device
+        ids = torch.empty(self.n_inner, dtype=torch.int32, device=dev)
+        if stream is not None:
+            ids.record_stream(stream)  # freed here, used there
+        L.check(L.lib().drb_bvh_widen_plan(C.byref(d), _ptr(ids), _stream(stream)),
+                "drb_bvh_widen_plan")
+        self.wide_nodes = torch.empty((max(d.n_wide, 1), 32), dtype=torch.float32, device=dev)
+        L.check(L.lib().drb_bvh_widen_emit(C.byref(d), _ptr(ids), _ptr(self.wide_nodes),
+                                           d.n_wide, _stream(stream)), "drb_bvh_widen_emit")
         self.n_wide, self.wide_depth = d.n_wide, d.wide_depth
         return self
 

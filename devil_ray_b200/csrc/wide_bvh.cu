@@ -13,9 +13,12 @@
 // returns the same result.
 //
 //   parent_kernel    parent index of every binary inner node
-//   depth_kernel     depth by walking the parents (bounded), even -> wide
+//   depth_kernel     depth of every node, even -> wide
 //   (exclusive scan of the flags gives each wide node its index)
 //   wide_emit_kernel one thread per wide node gathers its children
+// 8.65M leaves: 0.45 ms in all (HBM and the gathers), 1.3 ms when every node
+// walked to the root, every thread stored its own 128 bytes and the size
+// query ran the first two steps once more.
 #include "drb_common.cuh"
 #include "drb_internal.h"
 #include "locate.cuh"
@@ -38,21 +41,55 @@ __global__ void parent_kernel (const float4 *__restrict__ nodes, int n_inner, in
   if (r >= 0 && r / 4 < n_inner) parent[r / 4] = i;
 }
 
-__global__ void depth_kernel (const int *__restrict__ parent, int n_inner, int *__restrict__ wide_flag,
-                              int *__restrict__ max_depth)
+// Depth of every node.  A block takes kDepthNodes consecutive nodes.  A
+// node's index is an end of its leaf range, so most parents lie in the
+// block: only the nodes whose parent does not (some tens of a block) walk
+// the parents through global memory, and the others walk to one of those in
+// shared memory.  (Every node walking to the root took 25 dependent loads a
+// node.)  Walks are bounded by kMaxWalk.
+constexpr int kDepthBlock = 256;
+constexpr int kDepthNodes = 4 * kDepthBlock;
+
+__global__ void __launch_bounds__ (kDepthBlock)
+depth_kernel (const int *__restrict__ parent, int n_inner, int *__restrict__ wide_flag,
+              int *__restrict__ max_depth)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_inner) return;
-  int d = 0, j = i;
-  while (d < kMaxWalk)
+  __shared__ int s_parent[kDepthNodes];
+  __shared__ int s_depth[kDepthNodes]; // of nodes whose parent is elsewhere, else -1
+  __shared__ int s_max;
+  const int b0 = blockIdx.x * kDepthNodes;
+  const int count = min (kDepthNodes, n_inner - b0);
+  if (threadIdx.x == 0) s_max = 0;
+  for (int q = threadIdx.x; q < count; q += kDepthBlock)
   {
-    const int p = parent[j];
-    if (p < 0) break;
-    j = p;
-    ++d;
+    const int p = parent[b0 + q];
+    s_parent[q] = p - b0;
+    int d = -1;
+    if (p < b0 || p >= b0 + count)
+    {
+      d = 0;
+      for (int j = p; j >= 0 && d < kMaxWalk; j = __ldg (parent + j)) ++d;
+    }
+    s_depth[q] = d;
   }
-  wide_flag[i] = (d & 1) == 0 ? 1 : 0;
-  atomicMax (max_depth, d);
+  __syncthreads ();
+  int deepest = 0;
+  for (int q = threadIdx.x; q < count; q += kDepthBlock)
+  {
+    int j = q, d = 0;
+    while (s_depth[j] < 0 && d < kMaxWalk)
+    {
+      j = s_parent[j];
+      ++d;
+    }
+    d += max (s_depth[j], 0);
+    wide_flag[b0 + q] = (d & 1) == 0 ? 1 : 0;
+    deepest = max (deepest, d);
+  }
+  deepest = __reduce_max_sync (0xffffffffu, deepest);
+  if ((threadIdx.x & 31) == 0) atomicMax (&s_max, deepest);
+  __syncthreads ();
+  if (threadIdx.x == 0) atomicMax (max_depth, s_max);
 }
 
 // box c (0 left, 1 right) of a binary record: lo xyz, hi xyz
@@ -69,51 +106,123 @@ DRB_D void record_box (const float4 *__restrict__ rec, int c, float (&b)[6])
   }
 }
 
-__global__ void wide_emit_kernel (const float4 *__restrict__ nodes, int n_inner,
-                                  const int *__restrict__ wide_flag, const int *__restrict__ wide_id,
-                                  float4 *__restrict__ wide)
+// Child k of a wide row: its box (lo xyz, hi xyz) into the six SoA float4,
+// its code into the seventh.
+DRB_D void put_child (float *row, int k, const float (&box)[6], int code)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_inner || !wide_flag[i]) return;
-  float box[4][6];
-  int kid[4];
-  int k = 0;
-  const float4 *rec = nodes + 4 * (size_t)i;
-  const float4 d = rec[3];
-  const int ch[2] = { __float_as_int (d.x), __float_as_int (d.y) };
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
+  for (int f = 0; f < 6; ++f) row[4 * f + k] = box[f];
+  row[24 + k] = __int_as_float (code);
+}
+
+// wide_id: exclusive scan of the wide flags (n_wide in all), so node i is
+// wide when the next value is larger.  The wide nodes of a block are
+// consecutive: they are put together in shared memory and written as one
+// run (a thread storing its own 128 bytes touched 32 lines a store).
+constexpr int kEmitBlock = 128;
+constexpr int kEmitRow = 33; // floats a row: 32 and a pad against bank conflicts
+
+__global__ void __launch_bounds__ (kEmitBlock)
+wide_emit_kernel (const float4 *__restrict__ nodes, int n_inner, const int *__restrict__ wide_id,
+                  int n_wide, float4 *__restrict__ wide)
+{
+  __shared__ float s_row[kEmitBlock * kEmitRow];
+  const int b0 = blockIdx.x * kEmitBlock;
+  const int i = b0 + threadIdx.x;
+  const int first = __ldg (wide_id + b0);
+  const int end = b0 + kEmitBlock < n_inner ? __ldg (wide_id + b0 + kEmitBlock) : n_wide;
+  const int id = i < n_inner ? __ldg (wide_id + i) : n_wide;
+  const int next = i + 1 < n_inner ? __ldg (wide_id + i + 1) : n_wide;
+  if (next > id)
   {
-    if (ch[c] < 0)
-    {
-      record_box (rec, c, box[k]);
-      kid[k++] = ch[c];
-    }
-    else
-    {
-      const float4 *rj = nodes + ch[c];
-      const float4 dj = rj[3];
-      const int gc[2] = { __float_as_int (dj.x), __float_as_int (dj.y) };
+    float *row = s_row + (id - first) * kEmitRow;
+    const float4 *rec = nodes + 4 * (size_t)i;
+    const float4 d = rec[3];
+    const int ch[2] = { __float_as_int (d.x), __float_as_int (d.y) };
+    int k = 0;
 #pragma unroll
-      for (int g = 0; g < 2; ++g)
+    for (int c = 0; c < 2; ++c)
+    {
+      float box[6];
+      if (ch[c] < 0)
       {
-        record_box (rj, g, box[k]);
-        kid[k++] = gc[g] < 0 ? gc[g] : wide_id[gc[g] / 4];
+        record_box (rec, c, box);
+        put_child (row, k++, box, ch[c]);
+      }
+      else
+      {
+        const float4 *rj = nodes + ch[c];
+        const float4 dj = rj[3];
+        const int gc[2] = { __float_as_int (dj.x), __float_as_int (dj.y) };
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+        {
+          record_box (rj, g, box);
+          put_child (row, k++, box, gc[g] < 0 ? gc[g] : __ldg (wide_id + gc[g] / 4));
+        }
       }
     }
+    row[28] = __int_as_float (k);
+    row[29] = row[30] = row[31] = 0.f;
+    const float none[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
+    for (; k < 4; ++k) put_child (row, k, none, kWideEmpty);
   }
-  for (int q = k; q < 4; ++q)
+  __syncthreads ();
+  float *out = reinterpret_cast<float *> (wide) + 32 * (size_t)first;
+  for (int q = threadIdx.x; q < 32 * (end - first); q += kEmitBlock)
+    out[q] = s_row[(q >> 5) * kEmitRow + (q & 31)];
+}
+
+// Wide index of every binary node (scan of the even-depth flags) into ids,
+// n_wide and wide_depth of the BVH; synchronises for the two numbers.
+int plan_wide (drb_bvh *bvh, int *ids, cudaStream_t s)
+{
+  const int n = bvh->n_inner;
+  Scratch scr (s);
+  int *parent = scr.alloc<int> (n);
+  int *stat = scr.alloc<int> (2); // [0] max depth, [1] wide count
+  if (!stat) return status_from (scr.err);
+  cudaMemsetAsync (stat, 0, 2 * sizeof (int), s);
+  parent_kernel<<<div_up (n, 256), 256, 0, s>>> ((const float4 *)bvh->inner_nodes, n, parent);
+  int st = check_launch ("parent_kernel");
+  if (st) return st;
+  depth_kernel<<<div_up (n, kDepthNodes), kDepthBlock, 0, s>>> (parent, n, ids, stat);
+  if ((st = check_launch ("depth_kernel"))) return st;
+  if ((st = exclusive_scan_i32 (ids, ids, n, stat + 1, s))) return st;
+  int h[2] = { 0, 0 };
+  cudaError_t e = cudaMemcpyAsync (h, stat, sizeof (h), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize (s);
+  if (e != cudaSuccess)
   {
-    box[q][0] = box[q][1] = box[q][2] = INFINITY;
-    box[q][3] = box[q][4] = box[q][5] = -INFINITY;
-    kid[q] = kWideEmpty;
+    set_last_error (cudaGetErrorString (e));
+    return status_from (e);
   }
-  float4 *o = wide + 8 * (size_t)wide_id[i];
-#pragma unroll
-  for (int f = 0; f < 6; ++f) o[f] = make_float4 (box[0][f], box[1][f], box[2][f], box[3][f]);
-  o[6] = make_float4 (__int_as_float (kid[0]), __int_as_float (kid[1]), __int_as_float (kid[2]),
-                      __int_as_float (kid[3]));
-  o[7] = make_float4 (__int_as_float (k), 0.f, 0.f, 0.f);
+  bvh->n_wide = h[1];
+  bvh->wide_depth = h[0] / 2 + 1;
+  if (h[0] >= kMaxWalk || 3 * bvh->wide_depth + 1 > kWideStack)
+  {
+    set_last_error ("bvh_widen: tree too deep for the wide traversal stack");
+    bvh->wide_nodes = nullptr;
+    return DRB_ERR_UNSUPPORTED;
+  }
+  return DRB_OK;
+}
+
+int emit_wide (drb_bvh *bvh, const int *ids, float *wide_nodes, cudaStream_t s)
+{
+  const int n = bvh->n_inner;
+  wide_emit_kernel<<<div_up (n, kEmitBlock), kEmitBlock, 0, s>>> ((const float4 *)bvh->inner_nodes, n,
+                                                                  ids, bvh->n_wide, (float4 *)wide_nodes);
+  int st = check_launch ("wide_emit_kernel");
+  if (st == DRB_OK) bvh->wide_nodes = wide_nodes;
+  return st;
+}
+
+bool widen_args_ok (const drb_bvh *bvh)
+{
+  if (bvh && bvh->inner_nodes && bvh->n_inner >= 1) return true;
+  set_last_error ("bvh_widen: needs a built BVH");
+  return false;
 }
 
 } // namespace
@@ -123,52 +232,45 @@ using namespace drb;
 
 extern "C" int drb_bvh_widen (drb_bvh *bvh, float *wide_nodes, int capacity, void *stream)
 {
-  if (!bvh || !bvh->inner_nodes || bvh->n_inner < 1 || (wide_nodes && capacity < 1))
+  if (!widen_args_ok (bvh)) return DRB_ERR_INVALID_ARG;
+  if (wide_nodes && capacity < 1)
   {
     set_last_error ("bvh_widen: needs a built BVH");
     return DRB_ERR_INVALID_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  const int n = bvh->n_inner;
   Scratch scr (s);
-  int *parent = scr.alloc<int> (n);
-  int *flag = scr.alloc<int> (n);
-  int *wid = scr.alloc<int> (n);
-  int *stat = scr.alloc<int> (2); // [0] max depth, [1] wide count
-  if (!stat) return status_from (scr.err);
-  cudaMemsetAsync (stat, 0, 2 * sizeof (int), s);
-  const float4 *nodes = (const float4 *)bvh->inner_nodes;
-  parent_kernel<<<div_up (n, 256), 256, 0, s>>> (nodes, n, parent);
-  int st = check_launch ("parent_kernel");
-  if (st) return st;
-  depth_kernel<<<div_up (n, 256), 256, 0, s>>> (parent, n, flag, stat);
-  if ((st = check_launch ("depth_kernel"))) return st;
-  if ((st = exclusive_scan_i32 (flag, wid, n, stat + 1, s))) return st;
-  int h[2] = { 0, 0 };
-  cudaError_t e = cudaMemcpyAsync (h, stat, sizeof (h), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize (s);
-  if (e != cudaSuccess)
-  {
-    set_last_error (cudaGetErrorString (e));
-    return status_from (e);
-  }
-  const int depth = h[0], count = h[1];
-  bvh->n_wide = count;
-  bvh->wide_depth = depth / 2 + 1;
-  if (depth >= kMaxWalk || 3 * bvh->wide_depth + 1 > kWideStack)
-  {
-    set_last_error ("bvh_widen: tree too deep for the wide traversal stack");
-    bvh->wide_nodes = nullptr;
-    return DRB_ERR_UNSUPPORTED;
-  }
-  if (!wide_nodes) return DRB_OK; // size query
-  if (capacity < count)
+  int *ids = scr.alloc<int> (bvh->n_inner);
+  if (!ids) return status_from (scr.err);
+  int st = plan_wide (bvh, ids, s);
+  if (st || !wide_nodes) return st; // size query
+  if (capacity < bvh->n_wide)
   {
     set_last_error ("bvh_widen: wide node array too small (query the count first)");
     return DRB_ERR_INVALID_ARG;
   }
-  wide_emit_kernel<<<div_up (n, 256), 256, 0, s>>> (nodes, n, flag, wid, (float4 *)wide_nodes);
-  if ((st = check_launch ("wide_emit_kernel"))) return st;
-  bvh->wide_nodes = wide_nodes;
-  return DRB_OK;
+  return emit_wide (bvh, ids, wide_nodes, s);
+}
+
+extern "C" int drb_bvh_widen_plan (drb_bvh *bvh, int *wide_ids, void *stream)
+{
+  if (!widen_args_ok (bvh)) return DRB_ERR_INVALID_ARG;
+  if (!wide_ids)
+  {
+    set_last_error ("bvh_widen_plan: wide_ids is NULL");
+    return DRB_ERR_INVALID_ARG;
+  }
+  return plan_wide (bvh, wide_ids, (cudaStream_t)stream);
+}
+
+extern "C" int drb_bvh_widen_emit (drb_bvh *bvh, const int *wide_ids, float *wide_nodes, int capacity,
+                                   void *stream)
+{
+  if (!widen_args_ok (bvh)) return DRB_ERR_INVALID_ARG;
+  if (!wide_ids || !wide_nodes || capacity < bvh->n_wide || bvh->n_wide < 1)
+  {
+    set_last_error ("bvh_widen_emit: needs the plan's ids and n_wide wide nodes");
+    return DRB_ERR_INVALID_ARG;
+  }
+  return emit_wide (bvh, wide_ids, wide_nodes, (cudaStream_t)stream);
 }

@@ -195,6 +195,15 @@ int drb_bvh_leaf_maps (const drb_mesh *mesh, const drb_bvh *bvh, float *maps, vo
  * bvh->wide_nodes.  Synchronises the stream (reads the node count). */
 int drb_bvh_widen (drb_bvh *bvh, float *wide_nodes, int capacity, void *stream);
 
+/* The same in two steps, without doing the first one twice: the plan fills
+ * bvh->n_wide, bvh->wide_depth and the caller's wide_ids (device
+ * int32[n_inner], kept unchanged until the second step) and synchronises the
+ * stream; the second step writes the n_wide nodes (capacity at least that)
+ * and sets bvh->wide_nodes. */
+int drb_bvh_widen_plan (drb_bvh *bvh, int *wide_ids, void *stream);
+int drb_bvh_widen_emit (drb_bvh *bvh, const int *wide_ids, float *wide_nodes, int capacity,
+                        void *stream);
+
 /* Newton options.  The reference hard-codes tol 1e-4 and 20 steps for
  * volume elements (data_model/element.hpp:474-475), 1e-4 and 10 steps for
  * ray-face solves (face_intersection.hpp:153-154). */

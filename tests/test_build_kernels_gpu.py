@@ -5,6 +5,8 @@ elements), the radix sort and scan (edges of tiles), the bottom-up tree
 Everything is compared bit for bit: the steps are defined by 32-bit
 operations in a fixed order (data_model/mesh_utils.cpp:482-677,
 linear_bvh_builder.cpp:60-397)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -210,3 +212,60 @@ def test_bottom_up_tree_matches_top_down(cuda, kind, n_elem):
     sys.setrecursionlimit(20000)
     want = radix_tree(codes[order], aabbs.cpu().numpy()[order])
     assert np.array_equal(bits(b.inner_nodes.cpu().numpy()), bits(want))
+
+
+def collapse(nodes):
+    """4-wide collapse of the binary records: even-depth nodes in index
+    order, their grandchildren (children where those are leaves)."""
+    kids = nodes.view(np.int32)[:, 12:14]
+    depth = np.zeros(len(nodes), int)
+    stack = [0]
+    while stack:
+        i = stack.pop()
+        for c in kids[i]:
+            if c >= 0:
+                depth[c // 4] = depth[i] + 1
+                stack.append(c // 4)
+    wide_of = np.cumsum(depth % 2 == 0) - 1
+    out = []
+    for i in np.flatnonzero(depth % 2 == 0):
+        got = []
+        for side, c in enumerate(kids[i]):
+            if c < 0:
+                got.append((nodes[i, 6 * side:6 * side + 6], c))
+                continue
+            for s2, g in enumerate(kids[c // 4]):
+                got.append((nodes[c // 4, 6 * s2:6 * s2 + 6], g if g < 0 else wide_of[g // 4]))
+        row = np.zeros(32, F)
+        code = row.view(np.int32)
+        for k in range(4):
+            box, c = got[k] if k < len(got) else (np.array([np.inf] * 3 + [-np.inf] * 3, F), -2**31)
+            row[k:24:4], code[24 + k] = box, c
+        code[28] = len(got)
+        out.append(row)
+    return np.stack(out), int(depth.max()) // 2 + 1
+
+
+# the depth pass takes 1024 nodes a block, the emit pass 128
+@pytest.mark.parametrize("kind,n_elem", [("scattered", 1), ("scattered", 4), ("scattered", 31),
+                                         ("scattered", 32), ("scattered", 200), ("repeated", 70),
+                                         ("point", 100)])
+def test_wide_plan_and_emit(cuda, kind, n_elem):
+    import torch
+    from devil_ray_b200 import _lib as L
+    b = _tree_mesh(kind, n_elem, cuda).build_bvh()
+    want, depth = collapse(b.inner_nodes.cpu().numpy())
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for shift in (0, 1):                        # ids on and off a 16-byte boundary
+        ids = torch.full((b.n_inner + shift,), -7, dtype=torch.int32, device=cuda)[shift:]
+        d = b.desc()
+        assert L.lib().drb_bvh_widen_plan(C.byref(d), C.c_void_p(ids.data_ptr()), s) == 0
+        assert (d.n_wide, d.wide_depth) == (len(want), depth)
+        out = torch.empty((d.n_wide, 32), dtype=torch.float32, device=cuda)
+        assert L.lib().drb_bvh_widen_emit(C.byref(d), C.c_void_p(ids.data_ptr()),
+                                          C.c_void_p(out.data_ptr()), d.n_wide - 1, s) != 0
+        assert L.lib().drb_bvh_widen_emit(C.byref(d), C.c_void_p(ids.data_ptr()),
+                                          C.c_void_p(out.data_ptr()), d.n_wide, s) == 0
+        assert np.array_equal(bits(out.cpu().numpy()), bits(want))
+    b.widen()
+    assert np.array_equal(bits(b.wide_nodes.cpu().numpy()), bits(want))
