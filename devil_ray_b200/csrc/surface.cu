@@ -3,11 +3,15 @@
 //   MeshBoundary       extract_faces / sort_faces / unique_faces / reconstruct /
 //                      extract_face_dofs (data_model/mesh_utils.cpp:98-398,
 //                      filters/mesh_boundary.cpp:22-100).  The reference sorts
-//                      the (sorted) face corner tuples with a host std::sort;
-//                      here four stable radix passes on the tuple components
-//                      (least significant first) order them lexicographically
-//                      on the device.  Boundary faces have unique corner
-//                      tuples, so their order -- and the output -- is identical.
+//                      all (sorted) face corner tuples with a host std::sort
+//                      and drops those with an equal neighbour.  Here a hash
+//                      table finds the faces that occur once, and only those,
+//                      a few per cent, are put in the tuples' order (counting
+//                      sort on the smallest corner, ranks within its group).
+//                      Boundary faces have unique corner tuples, so their
+//                      order -- and the output -- is identical.
+//                      1.57M faces, 24,576 of them boundary, with the faces'
+//                      BVH: 1.53 -> 0.68 ms (the hash table's random access).
 //   intersect kernel   intersect_faces (rendering/surface.cpp:304-437): ordered
 //                      slab traversal (closer child first), per-leaf ray-face
 //                      Newton in (u, v, t) from the sub-box centre and t = near
@@ -28,6 +32,12 @@ namespace
 
 // ------------------------------------------------------------ boundary --
 
+// Largest group of boundary faces with one smallest corner that is ordered by
+// comparing its faces with one another (quadratic in the group); meshes with
+// a larger one (a vertex that hundreds of boundary faces share) take the
+// radix passes over the whole tuples.
+constexpr int kMaxFaceGroup = 128;
+
 DRB_D void sort4 (int (&f)[4])
 {
   // sorting network; the result equals the reference's sort4
@@ -39,7 +49,7 @@ DRB_D void sort4 (int (&f)[4])
 // extract_faces (Hex -> Tensor), mesh_utils.cpp:192-280: six sorted corner
 // tuples per element, face ids 0..5 = x, y, z, X, Y, Z.
 __global__ void extract_faces_kernel (const int *__restrict__ ctrl_idx, int n_elem, int p,
-                                      int4 *__restrict__ faces)
+                                      int4 *__restrict__ faces, int *__restrict__ keep)
 {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_elem) return;
@@ -55,6 +65,7 @@ __global__ void extract_faces_kernel (const int *__restrict__ ctrl_idx, int n_el
     int t[4] = { c[idx[f][0]], c[idx[f][1]], c[idx[f][2]], c[idx[f][3]] };
     sort4 (t);
     faces[(size_t)6 * e + f] = make_int4 (t[0], t[1], t[2], t[3]);
+    keep[(size_t)6 * e + f] = 1;
   }
 }
 
@@ -62,7 +73,7 @@ __global__ void extract_faces_kernel (const int *__restrict__ ctrl_idx, int n_el
 // triples per tet (fourth component -1), face f opposite corner f of
 // (u = 1, v = 1, w = 1, origin).
 __global__ void extract_tet_faces_kernel (const int *__restrict__ ctrl_idx, int n_elem, int p,
-                                          int4 *__restrict__ faces)
+                                          int4 *__restrict__ faces, int *__restrict__ keep)
 {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_elem) return;
@@ -79,7 +90,95 @@ __global__ void extract_tet_faces_kernel (const int *__restrict__ ctrl_idx, int 
     DRB_SWAP (0, 1) DRB_SWAP (1, 2) DRB_SWAP (0, 1)
 #undef DRB_SWAP
     faces[(size_t)4 * e + f] = make_int4 (t[0], t[1], t[2], -1);
+    keep[(size_t)4 * e + f] = 1;
   }
+}
+
+DRB_D bool same4 (int4 a, int4 b) { return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w; }
+DRB_D bool less4 (int4 a, int4 b)
+{
+  if (a.x != b.x) return (unsigned)a.x < (unsigned)b.x;
+  if (a.y != b.y) return (unsigned)a.y < (unsigned)b.y;
+  if (a.z != b.z) return (unsigned)a.z < (unsigned)b.z;
+  return (unsigned)a.w < (unsigned)b.w;
+}
+
+// unique_faces (mesh_utils.cpp:145-188): a face is on the boundary when no
+// other face has its corner tuple.  Open addressing over at least 2 n slots
+// (-1 empty) of face indices: the first face of a tuple takes a slot, every
+// later one finds it and marks both.  keep starts as ones.  A probe sequence
+// ends at an empty slot or an equal tuple, after `mask` probes at most.
+__global__ void face_match_kernel (const int4 *__restrict__ faces, int n, unsigned mask,
+                                   int *__restrict__ slots, int *__restrict__ keep)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int4 f = faces[i];
+  // multiplicative hashing (Knuth's golden-ratio constant), folding the
+  // high bits down after each component
+  unsigned h = 0u;
+  const int c[4] = { f.x, f.y, f.z, f.w };
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+  {
+    h = (h ^ (unsigned)c[k]) * 2654435769u;
+    h ^= h >> 15;
+  }
+  for (unsigned probe = 0; probe <= mask; ++probe)
+  {
+    int *slot = slots + ((h + probe) & mask);
+    const int other = atomicCAS (slot, -1, i);
+    if (other == -1) return;
+    if (same4 (faces[other], f))
+    {
+      keep[other] = 0;
+      keep[i] = 0;
+      return;
+    }
+  }
+}
+
+// Boundary faces per smallest corner, each face's arrival number in its
+// group; stats: the faces, the largest group, corners outside [0, n_ctrl).
+__global__ void __launch_bounds__ (256)
+face_count_kernel (const int4 *__restrict__ faces, const int *__restrict__ keep, int n, int n_ctrl,
+                   int *__restrict__ group, int *__restrict__ arrival, int *__restrict__ stats)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool on = i < n && keep[i];
+  int size = 0;
+  bool outside = false;
+  if (on)
+  {
+    const int c = faces[i].x;
+    outside = c < 0 || c >= n_ctrl;
+    if (!outside)
+    {
+      size = atomicAdd (group + c, 1) + 1;
+      arrival[i] = size - 1;
+    }
+  }
+  const unsigned all = __ballot_sync (0xffffffffu, on);
+  if (all == 0u) return;
+  const int largest = __reduce_max_sync (0xffffffffu, size);
+  const bool any_outside = __any_sync (0xffffffffu, outside);
+  if ((threadIdx.x & 31) == 0)
+  {
+    atomicAdd (stats, __popc (all));
+    atomicMax (stats + 1, largest);
+    if (any_outside) atomicMax (stats + 2, 1);
+  }
+}
+
+// list[place] = face, in group order (start: exclusive scan of the groups)
+// or, with start NULL, compacted (place: exclusive scan of keep).
+__global__ void face_place_kernel (const int4 *__restrict__ faces, const int *__restrict__ keep, int n,
+                                   const int *__restrict__ start, const int *__restrict__ place,
+                                   int *__restrict__ list)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n || !keep[i]) return;
+  list[(start ? start[faces[i].x] : 0) + place[i]] = i;
 }
 
 __global__ void face_key_kernel (const int4 *__restrict__ faces, const int *__restrict__ perm,
@@ -92,40 +191,40 @@ __global__ void face_key_kernel (const int4 *__restrict__ faces, const int *__re
   keys[i] = (unsigned)v;
 }
 
-__global__ void iota_kernel (int *a, int n)
+// The boundary faces in an order that keeps equal smallest corners together.
+struct FaceList
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = i;
-}
+  const int4 *faces; // corner tuples of all faces
+  const int *list;   // boundary faces
+  int n;
+  const int *start;  // first of each smallest corner's group, NULL: list is in order
+  int n_ctrl;
+};
 
-DRB_D bool same4 (int4 a, int4 b) { return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w; }
-
-// unique_faces (mesh_utils.cpp:145-188): a face is on the boundary when
-// neither sorted neighbour has the same tuple.
-__global__ void unique_flags_kernel (const int4 *__restrict__ faces, const int *__restrict__ perm,
-                                     int n, int *__restrict__ flags)
+// Place of the i-th listed face in the tuples' order.
+DRB_D int face_rank (const FaceList &fl, int i)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int4 me = faces[perm[i]];
-  bool dup = false;
-  if (i > 0 && same4 (me, faces[perm[i - 1]])) dup = true;
-  if (i < n - 1 && same4 (me, faces[perm[i + 1]])) dup = true;
-  flags[i] = dup ? 0 : 1;
+  if (!fl.start) return i;
+  const int4 me = fl.faces[fl.list[i]];
+  const int g0 = fl.start[me.x];
+  const int g1 = me.x + 1 < fl.n_ctrl ? fl.start[me.x + 1] : fl.n;
+  int rank = 0;
+  for (int q = g0; q < g1; ++q)
+    if (q != i && less4 (fl.faces[fl.list[q]], me)) ++rank;
+  return g0 + rank;
 }
 
 // reconstruct + extract_face_dofs (mesh_boundary.cpp:57-98): the quad's
 // (p+1)^2 dof indices into the unchanged volume value array.
-__global__ void face_dofs_kernel (const int *__restrict__ perm, const int *__restrict__ flags,
-                                  const int *__restrict__ offs, int n, int p,
-                                  const int *__restrict__ ctrl_idx, const int *__restrict__ field_idx,
+__global__ void face_dofs_kernel (FaceList fl, int p, const int *__restrict__ ctrl_idx,
+                                  const int *__restrict__ field_idx,
                                   int *__restrict__ out_idx, int *__restrict__ out_field_idx,
                                   int *__restrict__ elid_faceid)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !flags[i]) return;
-  const int face_idx = offs[i];
-  const int flat = perm[i];
+  if (i >= fl.n) return;
+  const int face_idx = face_rank (fl, i);
+  const int flat = fl.list[i];
   const int el = flat / 6;
   const int faceid = flat - 6 * el;
   const int e1 = p + 1, e2 = e1 * e1, e3 = e2 * e1;
@@ -158,16 +257,14 @@ __global__ void face_dofs_kernel (const int *__restrict__ perm, const int *__res
 // evaluators use (see lbvh.cu); here they come from the layered index, so
 // at order 1 the faces are the reference's and at orders 2-3 they are the
 // tets' own boundary.
-__global__ void tet_face_dofs_kernel (const int *__restrict__ perm, const int *__restrict__ flags,
-                                      const int *__restrict__ offs, int n, int p,
-                                      const int *__restrict__ ctrl_idx,
+__global__ void tet_face_dofs_kernel (FaceList fl, int p, const int *__restrict__ ctrl_idx,
                                       const int *__restrict__ field_idx, int *__restrict__ out_idx,
                                       int *__restrict__ out_field_idx, int *__restrict__ elid_faceid)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !flags[i]) return;
-  const int face_idx = offs[i];
-  const int flat = perm[i];
+  if (i >= fl.n) return;
+  const int face_idx = face_rank (fl, i);
+  const int flat = fl.list[i];
   const int el = flat / 4;
   const int faceid = flat - 4 * el;
   const int nd3 = tet_dofs (p), nd2 = tri_dofs (p);
@@ -746,56 +843,81 @@ extern "C" int drb_mesh_boundary (const drb_mesh *hex, const int *field_ctrl_idx
   cudaStream_t s = (cudaStream_t)stream;
   const int n = (int)nf;
   Scratch scr (s);
+  const int n_ctrl = hex->n_ctrl > 0 ? hex->n_ctrl : 0;
+  unsigned slots_n = 64;
+  while (slots_n < 2u * (unsigned)n && slots_n < (1u << 31)) slots_n *= 2u;
   int4 *faces = scr.alloc<int4> (n);
-  int *perm_a = scr.alloc<int> (n);
-  int *perm_b = scr.alloc<int> (n);
-  unsigned *keys = scr.alloc<unsigned> (n);
-  unsigned *keys_out = scr.alloc<unsigned> (n);
-  int *flags = scr.alloc<int> (n);
-  int *offs = scr.alloc<int> (n);
-  int *total = scr.alloc<int> (1);
+  int *keep = scr.alloc<int> (n);
+  int *slots = scr.alloc<int> (slots_n);
+  int *group = scr.alloc<int> ((size_t)n_ctrl + 1);
+  int *arrival = scr.alloc<int> (n);
+  int *stats = scr.alloc<int> (3);
   if (scr.err != cudaSuccess) return status_from (scr.err);
+  cudaMemsetAsync (slots, 0xff, sizeof (int) * (size_t)slots_n, s);
+  cudaMemsetAsync (group, 0, sizeof (int) * (size_t)n_ctrl, s);
+  cudaMemsetAsync (stats, 0, sizeof (int) * 3, s);
   if (tets)
-    extract_tet_faces_kernel<<<div_up (hex->n_elem, 128), 128, 0, s>>> (hex->ctrl_idx, hex->n_elem, hex->order, faces);
+    extract_tet_faces_kernel<<<div_up (hex->n_elem, 128), 128, 0, s>>> (hex->ctrl_idx, hex->n_elem, hex->order, faces, keep);
   else
-    extract_faces_kernel<<<div_up (hex->n_elem, 128), 128, 0, s>>> (hex->ctrl_idx, hex->n_elem, hex->order, faces);
+    extract_faces_kernel<<<div_up (hex->n_elem, 128), 128, 0, s>>> (hex->ctrl_idx, hex->n_elem, hex->order, faces, keep);
   int st = check_launch ("extract_faces_kernel");
   if (st) return st;
-  iota_kernel<<<div_up (n, 256), 256, 0, s>>> (perm_a, n);
-  if ((st = check_launch ("iota_kernel"))) return st;
-  // lexicographic order of (f0,f1,f2,f3): stable passes from the last key
-  for (int comp = 3; comp >= 0; --comp)
-  {
-    face_key_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, perm_a, n, comp, keys);
-    if ((st = check_launch ("face_key_kernel"))) return st;
-    if ((st = radix_sort_pairs (keys, perm_a, keys_out, perm_b, n, 32, s))) return st;
-    int *t = perm_a;
-    perm_a = perm_b;
-    perm_b = t;
-  }
-  unique_flags_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, perm_a, n, flags);
-  if ((st = check_launch ("unique_flags_kernel"))) return st;
-  if ((st = exclusive_scan_i32 (flags, offs, n, total, s))) return st;
-  int h = 0;
-  cudaError_t e = cudaMemcpyAsync (&h, total, sizeof (int), cudaMemcpyDeviceToHost, s);
+  face_match_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, n, slots_n - 1u, slots, keep);
+  if ((st = check_launch ("face_match_kernel"))) return st;
+  face_count_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, keep, n, n_ctrl, group, arrival, stats);
+  if ((st = check_launch ("face_count_kernel"))) return st;
+  int h[3] = { 0, 0, 0 };
+  cudaError_t e = cudaMemcpyAsync (h, stats, sizeof (h), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize (s);
   if (e != cudaSuccess) return status_from (e);
-  *n_faces = h;
-  if (face_ctrl_idx && tets)
+  const int nb = h[0];
+  *n_faces = nb;
+  if (!face_ctrl_idx || nb == 0) return DRB_OK;
+  FaceList fl;
+  fl.faces = faces;
+  fl.n = nb;
+  fl.n_ctrl = n_ctrl;
+  int *list = scr.alloc<int> (nb);
+  if (!list) return status_from (scr.err);
+  if (h[1] <= kMaxFaceGroup && !h[2])
   {
-    tet_face_dofs_kernel<<<div_up (n, 256), 256, 0, s>>> (perm_a, flags, offs, n, hex->order,
-                                                          hex->ctrl_idx, field_ctrl_idx,
-                                                          face_ctrl_idx, face_field_idx, elid_faceid);
-    if ((st = check_launch ("tet_face_dofs_kernel"))) return st;
+    if ((st = exclusive_scan_i32 (group, group, n_ctrl, nullptr, s))) return st;
+    face_place_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, keep, n, group, arrival, list);
+    if ((st = check_launch ("face_place_kernel"))) return st;
+    fl.list = list;
+    fl.start = group;
   }
-  else if (face_ctrl_idx)
+  else
   {
-    face_dofs_kernel<<<div_up (n, 256), 256, 0, s>>> (perm_a, flags, offs, n, hex->order,
-                                                      hex->ctrl_idx, field_ctrl_idx, face_ctrl_idx,
-                                                      face_field_idx, elid_faceid);
-    if ((st = check_launch ("face_dofs_kernel"))) return st;
+    // lexicographic order of (f0,f1,f2,f3): stable passes from the last key
+    int *other = scr.alloc<int> (nb);
+    unsigned *keys = scr.alloc<unsigned> (nb);
+    unsigned *keys_out = scr.alloc<unsigned> (nb);
+    if (scr.err != cudaSuccess) return status_from (scr.err);
+    if ((st = exclusive_scan_i32 (keep, arrival, n, nullptr, s))) return st;
+    face_place_kernel<<<div_up (n, 256), 256, 0, s>>> (faces, keep, n, nullptr, arrival, list);
+    if ((st = check_launch ("face_place_kernel"))) return st;
+    for (int comp = 3; comp >= 0; --comp)
+    {
+      face_key_kernel<<<div_up (nb, 256), 256, 0, s>>> (faces, list, nb, comp, keys);
+      if ((st = check_launch ("face_key_kernel"))) return st;
+      if ((st = radix_sort_pairs (keys, list, keys_out, other, nb, 32, s))) return st;
+      int *t = list;
+      list = other;
+      other = t;
+    }
+    fl.list = list;
+    fl.start = nullptr;
   }
-  return DRB_OK;
+  if (tets)
+  {
+    tet_face_dofs_kernel<<<div_up (nb, 128), 128, 0, s>>> (fl, hex->order, hex->ctrl_idx, field_ctrl_idx,
+                                                           face_ctrl_idx, face_field_idx, elid_faceid);
+    return check_launch ("tet_face_dofs_kernel");
+  }
+  face_dofs_kernel<<<div_up (nb, 128), 128, 0, s>>> (fl, hex->order, hex->ctrl_idx, field_ctrl_idx,
+                                                     face_ctrl_idx, face_field_idx, elid_faceid);
+  return check_launch ("face_dofs_kernel");
 }
 
 extern "C" int drb_surface_intersect (const drb_mesh *faces, const drb_bvh *bvh, const void *rays,
