@@ -7,11 +7,9 @@
 //
 // Tensor-core kernels (tcgen05 / UMMA, BF16 operands, FP32 accumulation in
 // tensor memory):
-//   gemm_kernel       D = A * B^T for A [M x K], B [N x K] (both K-major
-//                     bf16), one 128-row tile per CTA, K in chunks of 64,
-//                     optional split-K; fused epilogues: +bias & GELU
-//                     (storing the pre-activation), x GELU'(Z), fp32 store or
-//                     fp32 atomic accumulation (weight gradients)
+//   net_kernel        forward pass or a whole training step (forward, loss,
+//                     backward, weight gradients) per tile of 128 rows, one
+//                     launch; reduce_kernel adds the CTAs' gradients
 //   mlp_guess_kernel  fused inference: per tile of 128 (point, element)
 //                     pairs, features are built in shared memory, two UMMA
 //                     GEMMs run with the weights resident in shared memory,
@@ -215,266 +213,421 @@ __global__ void features_kernel (const float *__restrict__ packed, int stride,
   for (int k8 = 0; k8 < N::kInPad / 8; ++k8) dst[k8] = pair_features8<P> (row, pt, c, inv, k8);
 }
 
-// --------------------------------------------------------------- GEMM --
+// ---------------------------------------------- fused network evaluation --
+//
+// One kernel for the forward pass and for a training step.  A CTA of 16
+// warps takes tiles of 128 rows.  The activations of a tile never leave the
+// SM: the layer outputs are one accumulator of 128 TMEM columns, read by four
+// warpgroups (32 columns each, a thread per row), and every matrix operand
+// is a bf16 tile in shared memory that is used both ways, as it lies
+// (K-major) and transposed (MN-major), so no transposes are made:
+//   Z1 = X W1^T              H1 = gelu (Z1 + b1)
+//   Z2 = H1 W2^T             head, loss, dY, dZ2 = (W3^T dY) gelu'(Z2 + b2)
+//   dH1 = dZ2 W2             dZ1 = dH1 gelu'(Z1 + b1)
+//   dW2 += dZ2^T H1          dW1 += dZ1^T X
+// dW1 and dW2 stay in TMEM over the CTA's tiles; at its end every CTA
+// writes its sums to a slot of its own and reduce_kernel adds the slots in
+// order, so the gradients do not depend on the schedule.  The first form
+// (a GEMM kernel per product, 15 launches a step) kept Z and H in DRAM with
+// row-per-thread stores and transposed four matrices for the weight
+// gradients.
+// 16,384 rows at order 2: 27 us with the reduction, against 363; bound by
+// the chain of one tile per CTA (loads, four MMA groups, four epilogues).
 
-enum Epilogue
+struct NetArgs
 {
-  EPI_STORE = 0,     // C[r, c] = D (+ bias[c])                 fp32
-  EPI_BIAS_GELU = 1, // Z[r, c] = D + bias[c], H = bf16(gelu(Z))
-  EPI_GELU_GRAD = 2, // H[r, c] = bf16(D * gelu'(Z[r, c]))
-  EPI_ATOMIC = 3,    // atomicAdd(C[r * ldc + c], D) for c < ncols
-  EPI_ATOMIC_T = 4   // atomicAdd(C[c * ldc + r], D) for r < ncols (transposed)
-};
-
-struct GemmArgs
-{
-  const __nv_bfloat16 *A; // [M x K]
-  const __nv_bfloat16 *B; // [N x K]
-  int M, N, K;
-  int k_split;             // K elements per split (multiple of 64)
-  const float *bias;
-  float *C;                // fp32 output / pre-activation Z
-  __nv_bfloat16 *H;        // bf16 output
-  const float *Zin;        // pre-activation for EPI_GELU_GRAD
-  int ldc, ncols;          // for EPI_ATOMIC
+  const float *params;
+  const __nv_bfloat16 *wb;
+  const __nv_bfloat16 *X;
+  const float *target;
+  const float *weight;
+  int n, tiles;
+  float inv_count;
+  float *y_out;
+  float *partials; // partial_stride<P> () floats per CTA: the gradient, then the loss
   int *err;
 };
 
-constexpr int kKC = 64;       // K per chunk
-constexpr int kGemmN = 128;   // max N handled (TMEM columns)
+constexpr int kNetThreads = 512;
+constexpr int kNetGroups = 4; // warpgroups, 32 columns each
 
-template <int EPI>
-__global__ void __launch_bounds__ (128) gemm_kernel (GemmArgs g)
+template <int P> constexpr int partial_stride () { return (Net<P>::kParams + 1 + 3) / 4 * 4; }
+template <int P> constexpr size_t net_smem ()
 {
+  return (size_t)2 * 2 * 128 * Net<P>::kInPad + (size_t)3 * 2 * 128 * kHid;
+}
+static_assert (net_smem<1> () <= 200 * 1024 && net_smem<2> () <= 200 * 1024 &&
+               net_smem<3> () <= 200 * 1024, "the network's tiles fit beside the static arrays");
+static_assert (2 * kHid + Net<3>::kInPad <= 512, "accumulators fit in tensor memory");
+
+// Sums of 16 values over the warp's lanes: the sum of v[c] for c = lane & 15
+// (halving the columns a lane keeps at each step: 16 shuffles, not 80).
+DRB_D float column_sums (float (&v)[16], int lane)
+{
+#pragma unroll
+  for (int s = 8; s > 0; s >>= 1)
+#pragma unroll
+    for (int k = 0; k < s; ++k)
+    {
+      const bool upper = lane & s;
+      const float give = upper ? v[k] : v[k + s];
+      const float keep = upper ? v[k + s] : v[k];
+      v[k] = keep + __shfl_xor_sync (0xffffffffu, give, s);
+    }
+  return v[0] + __shfl_xor_sync (0xffffffffu, v[0], 16);
+}
+
+DRB_D uint32_t pack_bf16 (float a, float b)
+{
+  __nv_bfloat162 h = __floats2bfloat162_rn (a, b);
+  return *reinterpret_cast<uint32_t *> (&h);
+}
+
+// Columns [c0, c0 + 16) of a row of a 128-wide operand tile.
+DRB_D void store_row16 (unsigned char *tile, int row, int c0, const float (&v)[16])
+{
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    *reinterpret_cast<uint4 *> (tile + umma::tile_offset (row, c0 + 8 * q, kHid)) =
+    make_uint4 (pack_bf16 (v[8 * q], v[8 * q + 1]), pack_bf16 (v[8 * q + 2], v[8 * q + 3]),
+                pack_bf16 (v[8 * q + 4], v[8 * q + 5]), pack_bf16 (v[8 * q + 6], v[8 * q + 7]));
+}
+
+// A 128-row operand tile from row-major bf16 rows.  Consecutive lanes take
+// consecutive rows, so their 16-byte stores fill whole core matrices.
+template <int W> DRB_D void load_tile (unsigned char *tile, const __nv_bfloat16 *__restrict__ rows, int tid)
+{
+  for (int v = tid; v < 128 * (W / 8); v += kNetThreads)
+  {
+    const int r = v & 127, j = v >> 7;
+    *reinterpret_cast<uint4 *> (tile + umma::tile_offset (r, 8 * j, W)) =
+    __ldg (reinterpret_cast<const uint4 *> (rows + (size_t)r * W) + j);
+  }
+}
+
+template <int P, bool TRAIN>
+__global__ void __launch_bounds__ (kNetThreads, 1) net_kernel (NetArgs a)
+{
+  using N = Net<P>;
+  constexpr int kInPad = N::kInPad;
   extern __shared__ __align__ (1024) unsigned char smem[];
-  unsigned char *sA = smem;                       // 128 x 64 bf16 = 16 KB
-  unsigned char *sB = smem + 128 * kKC * 2;       // N x 64 bf16 <= 16 KB
+  unsigned char *sX = smem;
+  unsigned char *sW1 = sX + 2 * 128 * kInPad;
+  unsigned char *sW2 = sW1 + 2 * 128 * kInPad;
+  unsigned char *sH = sW2 + 2 * 128 * kHid; // H1, then dZ1
+  unsigned char *sZ = sH + 2 * 128 * kHid;  // dZ2
+  __shared__ float s_b1[kHid], s_b2[kHid], s_w3[kOut * kHid], s_b3[kOut];
+  __shared__ float s_y[kNetGroups][128][kOut];
+  __shared__ float s_sum[kNetThreads / 32][5][32];
   __shared__ __align__ (8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int m0 = blockIdx.x * 128;
-  const int kbeg = blockIdx.y * g.k_split;
-  const int kend = min (g.K, kbeg + g.k_split);
-  if (warp == 0) umma::tmem_alloc (&tmem_base, kGemmN);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = warp >> 2;   // this warpgroup's columns: [32 g, 32 g + 32)
+  const int row = tid & 127; // this thread's row = TMEM lane
+  load_tile<kInPad> (sW1, a.wb + N::kBW1, tid);
+  load_tile<kHid> (sW2, a.wb + N::kBW2, tid);
+  if (tid < kHid)
+  {
+    s_b1[tid] = a.params[N::kB1 + tid];
+    s_b2[tid] = a.params[N::kB2 + tid];
+  }
+  if (tid < kOut * kHid) s_w3[tid] = a.params[N::kW3 + tid];
+  if (tid < kOut) s_b3[tid] = a.params[N::kB3 + tid];
+  if (warp == 0) umma::tmem_alloc (&tmem_base, 512);
   if (tid == 0) umma::mbar_init (&mbar, 1);
   umma::fence_before_sync ();
   __syncthreads ();
   umma::fence_after_sync ();
-  const uint32_t tbase = tmem_base;
-  const uint32_t idesc = umma::idesc_bf16_f32 (128, g.N);
+  const uint32_t tD = tmem_base, tW2 = tD + kHid, tW1 = tD + 2 * kHid;
+  const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t tmine = tD + lane_off + 32 * g;
+  const uint32_t aX = umma::smem_addr (sX), aW1 = umma::smem_addr (sW1), aW2 = umma::smem_addr (sW2),
+                 aH = umma::smem_addr (sH), aZ = umma::smem_addr (sZ);
+  constexpr uint32_t kD = umma::idesc_bf16_f32 (128, kHid);
   uint32_t phase = 0;
   bool ok = true;
-  int chunks = 0;
-  for (int k0 = kbeg; k0 < kend; k0 += kKC)
+  // running column sums: dZ2 and the three dY x H2 products, then dZ1, per
+  // 16-column half (this lane's column is lane & 15)
+  float sums[2][5] = { { 0.f, 0.f, 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f, 0.f, 0.f } };
+  float db3[kOut] = { 0.f, 0.f, 0.f };
+  float loss = 0.f;
+  bool first = true;
+
+  for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x)
   {
-    // cooperative 16-byte loads into the interleaved layout
-    for (int v = tid; v < 128 * (kKC / 8); v += 128)
-    {
-      const int r = v / (kKC / 8), j = v - r * (kKC / 8);
-      const int k = k0 + 8 * j;
-      uint4 val = make_uint4 (0, 0, 0, 0);
-      if (m0 + r < g.M && k < kend)
-        val = *reinterpret_cast<const uint4 *> (g.A + (size_t)(m0 + r) * g.K + k);
-      *reinterpret_cast<uint4 *> (sA + umma::tile_offset (r, 8 * j, kKC)) = val;
-    }
-    for (int v = tid; v < g.N * (kKC / 8); v += 128)
-    {
-      const int r = v / (kKC / 8), j = v - r * (kKC / 8);
-      const int k = k0 + 8 * j;
-      uint4 val = make_uint4 (0, 0, 0, 0);
-      if (k < kend) val = *reinterpret_cast<const uint4 *> (g.B + (size_t)r * g.K + k);
-      *reinterpret_cast<uint4 *> (sB + umma::tile_offset (r, 8 * j, kKC)) = val;
-    }
+    const int i = tile * 128 + row;
+    load_tile<kInPad> (sX, a.X + (size_t)tile * 128 * kInPad, tid);
     umma::fence_async_smem ();
     __syncthreads ();
     if (tid == 0)
     {
       umma::fence_after_sync ();
-      const uint32_t a0 = umma::smem_addr (sA), b0 = umma::smem_addr (sB);
 #pragma unroll
-      for (int kk = 0; kk < kKC / 16; ++kk)
-      {
-        const uint64_t ad = umma::desc_kmajor (a0 + kk * 256, 128, (kKC / 8) * 128);
-        const uint64_t bd = umma::desc_kmajor (b0 + kk * 256, 128, (kKC / 8) * 128);
-        umma::mma_bf16 (tbase, ad, bd, idesc, (chunks > 0 || kk > 0) ? 1u : 0u);
-      }
+      for (int kk = 0; kk < kInPad / 16; ++kk)
+        umma::mma_bf16 (tD, umma::desc_rows (aX, kInPad, kk), umma::desc_rows (aW1, kInPad, kk), kD,
+                        kk > 0 ? 1u : 0u);
       umma::mma_commit (&mbar);
     }
-    ok = umma::mbar_wait (&mbar, phase, kWaitTries) && ok;
+    ok = __syncthreads_and (umma::mbar_wait (&mbar, phase, kWaitTries));
     phase ^= 1u;
-    ++chunks;
     umma::fence_after_sync ();
-    __syncthreads ();
-    if (!__syncthreads_and (ok)) break;
-  }
-  ok = __syncthreads_and (ok) != 0; // CTA-uniform before the warp-collective loads
-  if (!ok && tid == 0 && g.err) atomicExch (g.err, 1);
-  // epilogue: thread t owns accumulator row t (TMEM lane t)
-  const int r = m0 + tid;
-  if (ok && chunks > 0)
-  {
-    for (int c0 = 0; c0 < g.N; c0 += 32)
-    {
-      float d[32];
-      umma::tmem_ld32 (tbase + ((uint32_t)(warp * 32) << 16) + c0, d);
-      if (r >= g.M) continue;
+    if (!ok) break;
+    // H1 = gelu (Z1 + b1); gelu'(Z1 + b1) is kept for the backward pass
+    float dg1[2][16];
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
+    for (int half = 0; half < 2; ++half)
+    {
+      const int c0 = 32 * g + 16 * half;
+      float d[16];
+      umma::tmem_ld16 (tmine + 16 * half, d);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
       {
-        const int c = c0 + j;
-        if (c >= g.N) break;
-        if (EPI == EPI_STORE)
-          g.C[(size_t)r * g.N + c] = d[j] + (g.bias ? g.bias[c] : 0.f);
-        else if (EPI == EPI_BIAS_GELU)
-        {
-          const float z = d[j] + g.bias[c];
-          g.C[(size_t)r * g.N + c] = z;
-          g.H[(size_t)r * g.N + c] = __float2bfloat16_rn (gelu (z));
-        }
-        else if (EPI == EPI_GELU_GRAD)
-          g.H[(size_t)r * g.N + c] = __float2bfloat16_rn (d[j] * gelu_grad (g.Zin[(size_t)r * g.N + c]));
-        else if (EPI == EPI_ATOMIC)
-        {
-          if (c < g.ncols) atomicAdd (g.C + (size_t)r * g.ldc + c, d[j]);
-        }
-        else if (r < g.ncols)
-          atomicAdd (g.C + (size_t)c * g.ldc + r, d[j]);
+        const float z = d[j] + s_b1[c0 + j];
+        d[j] = gelu (z);
+        if (TRAIN) dg1[half][j] = gelu_grad (z);
       }
+      store_row16 (sH, row, c0, d);
+    }
+    umma::fence_async_smem ();
+    umma::fence_before_sync ();
+    __syncthreads ();
+    if (tid == 0)
+    {
+      umma::fence_after_sync ();
+#pragma unroll
+      for (int kk = 0; kk < kHid / 16; ++kk)
+        umma::mma_bf16 (tD, umma::desc_rows (aH, kHid, kk), umma::desc_rows (aW2, kHid, kk), kD,
+                        kk > 0 ? 1u : 0u);
+      umma::mma_commit (&mbar);
+    }
+    ok = __syncthreads_and (umma::mbar_wait (&mbar, phase, kWaitTries));
+    phase ^= 1u;
+    umma::fence_after_sync ();
+    if (!ok) break;
+    // head: y = W3 gelu (Z2 + b2) + b3, a part per warpgroup
+    float y[kOut] = { 0.f, 0.f, 0.f };
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+    {
+      const int c0 = 32 * g + 16 * half;
+      float d[16];
+      umma::tmem_ld16 (tmine + 16 * half, d);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+      {
+        const float h = gelu (d[j] + s_b2[c0 + j]);
+#pragma unroll
+        for (int o = 0; o < kOut; ++o) y[o] = fmaf (s_w3[o * kHid + c0 + j], h, y[o]);
+      }
+    }
+#pragma unroll
+    for (int o = 0; o < kOut; ++o) s_y[g][row][o] = y[o];
+    __syncthreads ();
+    const float w = TRAIN && i < a.n ? (a.weight ? __ldg (a.weight + i) : 1.f) : 0.f;
+    float dy[kOut];
+#pragma unroll
+    for (int o = 0; o < kOut; ++o)
+    {
+      const float yo = ((s_y[0][row][o] + s_y[1][row][o]) + (s_y[2][row][o] + s_y[3][row][o])) + s_b3[o];
+      const float e = TRAIN && i < a.n ? yo - __ldg (a.target + 3 * (size_t)i + o) : 0.f;
+      dy[o] = 2.f * w * e * a.inv_count;
+      if (g == 0)
+      {
+        loss += w * e * e * a.inv_count;
+        db3[o] += dy[o];
+        if (!TRAIN && i < a.n) a.y_out[3 * (size_t)i + o] = yo;
+      }
+    }
+    if (TRAIN)
+    {
+      // dZ2 and its sums
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+      {
+        const int c0 = 32 * g + 16 * half;
+        float h[16], v[16];
+        umma::tmem_ld16 (tmine + 16 * half, h);
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+        {
+          const float z = h[j] + s_b2[c0 + j];
+          float dh = 0.f;
+#pragma unroll
+          for (int o = 0; o < kOut; ++o) dh = fmaf (s_w3[o * kHid + c0 + j], dy[o], dh);
+          v[j] = dh * gelu_grad (z);
+          h[j] = gelu (z);
+        }
+        store_row16 (sZ, row, c0, v);
+        sums[half][0] += column_sums (v, lane);
+#pragma unroll
+        for (int o = 0; o < kOut; ++o)
+        {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = dy[o] * h[j];
+          sums[half][1 + o] += column_sums (v, lane);
+        }
+      }
+      umma::fence_async_smem ();
+      umma::fence_before_sync ();
+      __syncthreads ();
+      if (tid == 0)
+      {
+        umma::fence_after_sync ();
+#pragma unroll
+        for (int kk = 0; kk < kHid / 16; ++kk)
+          umma::mma_bf16 (tD, umma::desc_rows (aZ, kHid, kk), umma::desc_cols (aW2, kHid, kk),
+                          umma::idesc_bf16_f32 (128, kHid, false, true), kk > 0 ? 1u : 0u);
+#pragma unroll
+        for (int kk = 0; kk < 128 / 16; ++kk)
+          umma::mma_bf16 (tW2, umma::desc_cols (aZ, kHid, kk), umma::desc_cols (aH, kHid, kk),
+                          umma::idesc_bf16_f32 (128, kHid, true, true), first && kk == 0 ? 0u : 1u);
+        umma::mma_commit (&mbar);
+      }
+      ok = __syncthreads_and (umma::mbar_wait (&mbar, phase, kWaitTries));
+      phase ^= 1u;
+      umma::fence_after_sync ();
+      if (!ok) break;
+      // dZ1 over H1, which dW2 has read
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+      {
+        const int c0 = 32 * g + 16 * half;
+        float d[16];
+        umma::tmem_ld16 (tmine + 16 * half, d);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[j] *= dg1[half][j];
+        store_row16 (sH, row, c0, d);
+        sums[half][4] += column_sums (d, lane);
+      }
+      umma::fence_async_smem ();
+      umma::fence_before_sync ();
+      __syncthreads ();
+      if (tid == 0)
+      {
+        umma::fence_after_sync ();
+#pragma unroll
+        for (int kk = 0; kk < 128 / 16; ++kk)
+          umma::mma_bf16 (tW1, umma::desc_cols (aH, kHid, kk), umma::desc_cols (aX, kInPad, kk),
+                          umma::idesc_bf16_f32 (128, kInPad, true, true), first && kk == 0 ? 0u : 1u);
+        umma::mma_commit (&mbar);
+      }
+      ok = __syncthreads_and (umma::mbar_wait (&mbar, phase, kWaitTries));
+      phase ^= 1u;
+      umma::fence_after_sync ();
+      if (!ok) break;
+    }
+    else
+    {
+      // the next tile writes s_y and the accumulator again
+      umma::fence_before_sync ();
+      __syncthreads ();
+      umma::fence_after_sync ();
+    }
+    first = false;
+  }
+  if (!ok && tid == 0 && a.err) atomicExch (a.err, 1);
+  if (TRAIN)
+  {
+    // this CTA's sums to its slot (zeros where a wait ran out)
+    float *out = a.partials + (size_t)blockIdx.x * partial_stride<P> ();
+#pragma unroll 1
+    for (int c0 = 32 * g; c0 < kHid + kInPad; c0 += 32 * kNetGroups)
+    {
+      // W2's columns, then W1's
+      float d[32];
+      umma::tmem_ld32 (tW2 + lane_off + c0, d);
+      const bool w2 = c0 < kHid;
+      float *dst = out + (w2 ? N::kW2 + row * kHid + c0 : N::kW1 + row * N::kIn + c0 - kHid);
+      const int limit = w2 ? 32 : min (32, N::kIn - (c0 - kHid));
+      if (w2 || N::kIn % 4 == 0) // 16-byte aligned: every offset is a multiple of 4
+      {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          if (j < limit)
+            *reinterpret_cast<float4 *> (dst + j) =
+            ok ? make_float4 (d[j], d[j + 1], d[j + 2], d[j + 3]) : make_float4 (0.f, 0.f, 0.f, 0.f);
+      }
+      else
+      {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j < limit) dst[j] = ok ? d[j] : 0.f;
+      }
+    }
+    // sums over the four warps of a warpgroup, rows in order
+#pragma unroll
+    for (int q = 0; q < 5; ++q) s_sum[warp][q][lane] = lane < 16 ? sums[0][q] : sums[1][q];
+    float *s_tail = &s_y[0][0][0]; // loss, db3 per warp of group 0
+    __syncthreads ();
+    if (g == 0)
+    {
+      float t[4] = { loss, db3[0], db3[1], db3[2] };
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+      {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_xor_sync (0xffffffffu, t[q], o);
+        if (lane == 0) s_tail[4 * warp + q] = t[q];
+      }
+    }
+    __syncthreads ();
+    if (tid < kHid)
+    {
+      const int w0 = 4 * (tid >> 5); // the warps that hold this column
+      float t[5];
+#pragma unroll
+      for (int q = 0; q < 5; ++q)
+        t[q] = (s_sum[w0][q][lane] + s_sum[w0 + 1][q][lane]) + (s_sum[w0 + 2][q][lane] + s_sum[w0 + 3][q][lane]);
+      out[N::kB2 + tid] = t[0];
+#pragma unroll
+      for (int o = 0; o < kOut; ++o) out[N::kW3 + o * kHid + tid] = t[1 + o];
+      out[N::kB1 + tid] = t[4];
+    }
+    if (tid < 4)
+    {
+      const float t = (s_tail[tid] + s_tail[4 + tid]) + (s_tail[8 + tid] + s_tail[12 + tid]);
+      out[tid == 0 ? N::kParams : N::kB3 + tid - 1] = t;
     }
   }
   umma::fence_before_sync ();
   __syncthreads ();
-  if (warp == 0) umma::tmem_dealloc (tbase, kGemmN);
+  if (warp == 0) umma::tmem_dealloc (tmem_base, 512);
 }
 
-// ------------------------------------------------------- head / losses --
-
-// y = W3 gelu(Z2) + b3; masked MSE; dY; grads of W3, b3; dZ2 = (W3^T dY) x
-// gelu'(Z2) as bf16; db2.  One block of 128 threads per 128 rows, in two
-// coalesced phases: a warp per row for the head and dY (Z2 rows read as
-// float4, the 3 dot products reduced by shuffles), then a thread per column
-// over the block's rows for dZ2 and the weight-gradient column sums, so the
-// block adds one partial per parameter to the global gradient.
-template <int P>
-__global__ void __launch_bounds__ (128)
-head_kernel (const float *__restrict__ p, const float *__restrict__ Z2, const float *__restrict__ target,
-             const float *__restrict__ weight, int n, int n_pad, float inv_count, float *__restrict__ y_out,
-             float *__restrict__ grad, __nv_bfloat16 *__restrict__ dZ2, float *__restrict__ loss)
+// Gradient and loss: the sum of the CTAs' slots.  A block takes 128
+// consecutive values; 32 threads read them as float4, 8 rows of threads
+// share the slots.
+__global__ void __launch_bounds__ (256)
+reduce_kernel (const float *__restrict__ partials, int slots, int stride, int n_params,
+               float *__restrict__ grad, float *__restrict__ loss)
 {
-  constexpr int kW3 = Net<P>::kW3, kB3 = Net<P>::kB3, kB2 = Net<P>::kB2;
-  __shared__ float s_w3[kOut * kHid];
-  __shared__ float s_dy[128][kOut];
-  __shared__ float s_loss;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int q = tid; q < kOut * kHid; q += blockDim.x) s_w3[q] = p[kW3 + q];
-  if (tid == 0) s_loss = 0.f;
-  __syncthreads ();
-  const int r0 = blockIdx.x * 128;
-  const int rows = min (128, n_pad - r0);
-  const float b3[kOut] = { p[kB3], p[kB3 + 1], p[kB3 + 2] };
-  // phase 1: head and dY, a warp per row, lane l holds columns [4 l, 4 l + 4)
-  for (int rr = warp; rr < rows; rr += 4)
+  __shared__ float4 s[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int at = blockIdx.x * 128 + 4 * tx;
+  float4 acc = make_float4 (0.f, 0.f, 0.f, 0.f);
+  if (at < stride)
   {
-    const int i = r0 + rr;
-    const float4 z4 = *reinterpret_cast<const float4 *> (Z2 + (size_t)i * kHid + 4 * lane);
-    const float z[4] = { z4.x, z4.y, z4.z, z4.w };
-    float y[kOut] = { 0.f, 0.f, 0.f };
-#pragma unroll
-    for (int t = 0; t < 4; ++t)
+#pragma unroll 8
+    for (int q = ty; q < slots; q += 8)
     {
-      const float h = gelu (z[t]);
-#pragma unroll
-      for (int o = 0; o < kOut; ++o) y[o] = fmaf (s_w3[o * kHid + 4 * lane + t], h, y[o]);
-    }
-#pragma unroll
-    for (int o = 0; o < kOut; ++o)
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) y[o] += __shfl_xor_sync (0xffffffffu, y[o], off);
-    if (lane == 0)
-    {
-      const float w = (i < n && weight) ? weight[i] : (i < n ? 1.f : 0.f);
-      float l = 0.f;
-#pragma unroll
-      for (int o = 0; o < kOut; ++o)
-      {
-        const float yo = y[o] + b3[o];
-        const float e = (i < n && target) ? (yo - target[3 * (size_t)i + o]) : 0.f;
-        l += w * e * e;
-        s_dy[rr][o] = 2.f * w * e * inv_count;
-        if (y_out && i < n) y_out[3 * (size_t)i + o] = yo;
-      }
-      if (grad) atomicAdd (&s_loss, l * inv_count);
+      const float4 v = __ldg (reinterpret_cast<const float4 *> (partials + (size_t)q * stride + at));
+      acc.x += v.x;
+      acc.y += v.y;
+      acc.z += v.z;
+      acc.w += v.w;
     }
   }
-  if (!grad) return;
+  s[ty][tx] = acc;
   __syncthreads ();
-  // phase 2: thread c owns column c of the block's rows
-  const int c = tid;
-  float gw3[kOut] = { 0.f, 0.f, 0.f };
-  float db2 = 0.f;
-  const float w3c[kOut] = { s_w3[c], s_w3[kHid + c], s_w3[2 * kHid + c] };
-  for (int rr = 0; rr < rows; ++rr)
+  if (threadIdx.x < 128)
   {
-    const size_t at = (size_t)(r0 + rr) * kHid + c;
-    const float z = Z2[at];
-    const float h = gelu (z);
-    float dh = 0.f;
+    const int v = blockIdx.x * 128 + threadIdx.x;
+    float t = 0.f;
 #pragma unroll
-    for (int o = 0; o < kOut; ++o)
-    {
-      const float dy = s_dy[rr][o];
-      gw3[o] = fmaf (dy, h, gw3[o]);
-      dh = fmaf (w3c[o], dy, dh);
-    }
-    const float dz = dh * gelu_grad (z);
-    dZ2[at] = __float2bfloat16_rn (dz);
-    db2 += dz;
-  }
-#pragma unroll
-  for (int o = 0; o < kOut; ++o) atomicAdd (grad + kW3 + o * kHid + c, gw3[o]);
-  atomicAdd (grad + kB2 + c, db2);
-  if (tid < kOut)
-  {
-    float gb = 0.f;
-    for (int rr = 0; rr < rows; ++rr) gb += s_dy[rr][tid];
-    atomicAdd (grad + kB3 + tid, gb);
-  }
-  if (tid == 0 && loss) atomicAdd (loss, s_loss);
-}
-
-// column sums of a bf16 [rows x 128] matrix into grad[off + c]
-__global__ void colsum_kernel (const __nv_bfloat16 *__restrict__ M, int rows, float *__restrict__ out)
-{
-  __shared__ float s[kHid];
-  if (threadIdx.x < kHid) s[threadIdx.x] = 0.f;
-  __syncthreads ();
-  const int c = threadIdx.x & (kHid - 1);
-  float acc = 0.f;
-  for (int r = blockIdx.x * (blockDim.x / kHid) + threadIdx.x / kHid; r < rows;
-       r += gridDim.x * (blockDim.x / kHid))
-    acc += __bfloat162float (M[(size_t)r * kHid + c]);
-  atomicAdd (&s[c], acc);
-  __syncthreads ();
-  if (threadIdx.x < kHid) atomicAdd (out + threadIdx.x, s[threadIdx.x]);
-}
-
-// bf16 transpose [rows x cols] -> [cols x rows]
-__global__ void transpose_kernel (const __nv_bfloat16 *__restrict__ in, int rows, int cols,
-                                  __nv_bfloat16 *__restrict__ out)
-{
-  __shared__ __nv_bfloat16 t[32][33];
-  const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y)
-  {
-    const int r = by + j, c = bx + threadIdx.x;
-    t[j][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * cols + c] : __float2bfloat16_rn (0.f);
-  }
-  __syncthreads ();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y)
-  {
-    const int c = bx + j, r = by + threadIdx.x;
-    if (c < cols && r < rows) out[(size_t)c * rows + r] = t[threadIdx.x][j];
+    for (int q = 0; q < 8; ++q) t += reinterpret_cast<const float *> (s[q])[threadIdx.x];
+    if (v < n_params) grad[v] = t;
+    else if (v == n_params && loss) loss[0] = t;
   }
 }
 
@@ -709,17 +862,6 @@ __global__ void __launch_bounds__ (128 * Net<P>::kGroups, 1) mlp_guess_kernel (G
   if (warp == 0) umma::tmem_dealloc (tmem_base, kGuessGroups * kHid);
 }
 
-template <int EPI> int launch_gemm (const GemmArgs &g, cudaStream_t s)
-{
-  const size_t smem = (size_t)128 * kKC * 2 + (size_t)kGemmN * kKC * 2;
-  // at most 4 CTAs per SM so that their TMEM (128 columns each) always fits
-  const size_t smem_req = smem < 48 * 1024 ? 48 * 1024 : smem;
-  cudaFuncSetAttribute (gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_req);
-  dim3 grid ((unsigned)div_up (g.M, 128), (unsigned)div_up (g.K, g.k_split));
-  gemm_kernel<EPI><<<grid, 128, smem_req, s>>> (g);
-  return check_launch ("gemm_kernel");
-}
-
 } // namespace mlp
 } // namespace drb
 
@@ -752,56 +894,36 @@ int features_p (const drb_mesh *mesh, const int *elem, const float *pts, int n, 
   return check_launch ("features_kernel");
 }
 
+// Slots of a training step: one per CTA of net_kernel.
+int net_ctas (int n_pad) { return min (n_pad / 128, sm_count ()); }
+
+// Large enough for every device's slots: a tile has one CTA at most.
 template <int P> long long workspace_p (int n_pad)
 {
-  const long long r = n_pad;
-  return r * kHid * 4 * 2 + r * kHid * 2 * 4 + r * kHid * 2 * 3 + r * Net<P>::kInPad * 2 + 4096;
+  return (long long)(n_pad / 128) * partial_stride<P> () * 4 + 4096;
 }
 
-// The two layers of the forward pass into Z1/H1 and Z2/H2.
-template <int P>
-int forward_layers (const float *params, const __nv_bfloat16 *wb, const void *X, int n_pad,
-                    float *Z1, __nv_bfloat16 *H1, float *Z2, __nv_bfloat16 *H2, int *err,
-                    cudaStream_t s)
+template <int P, bool TRAIN> int launch_net (const NetArgs &a, int ctas, cudaStream_t s)
 {
-  using N = Net<P>;
-  GemmArgs g{};
-  g.A = (const __nv_bfloat16 *)X;
-  g.B = wb + N::kBW1;
-  g.M = n_pad;
-  g.N = kHid;
-  g.K = N::kInPad;
-  g.k_split = ((N::kInPad + kKC - 1) / kKC) * kKC;
-  g.bias = params + N::kB1;
-  g.C = Z1;
-  g.H = H1;
-  g.err = err;
-  int st = launch_gemm<EPI_BIAS_GELU> (g, s);
-  if (st) return st;
-  g.A = H1;
-  g.B = wb + N::kBW2;
-  g.K = kHid;
-  g.k_split = kHid;
-  g.bias = params + N::kB2;
-  g.C = Z2;
-  g.H = H2;
-  return launch_gemm<EPI_BIAS_GELU> (g, s);
+  constexpr size_t smem = net_smem<P> ();
+  cudaFuncSetAttribute (net_kernel<P, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  net_kernel<P, TRAIN><<<ctas, kNetThreads, smem, s>>> (a);
+  return check_launch ("net_kernel");
 }
 
 template <int P>
 int forward_p (const float *params, const void *wbf16, const void *X, int n, int n_pad, float *y,
-               void *workspace, int *err, cudaStream_t s)
+               int *err, cudaStream_t s)
 {
-  unsigned char *w = (unsigned char *)workspace;
-  float *Z1 = (float *)w;
-  float *Z2 = Z1 + (size_t)n_pad * kHid;
-  __nv_bfloat16 *H1 = (__nv_bfloat16 *)(Z2 + (size_t)n_pad * kHid);
-  __nv_bfloat16 *H2 = H1 + (size_t)n_pad * kHid;
-  int st = forward_layers<P> (params, (const __nv_bfloat16 *)wbf16, X, n_pad, Z1, H1, Z2, H2, err, s);
-  if (st) return st;
-  head_kernel<P><<<div_up (n_pad, 128), 128, 0, s>>> (params, Z2, nullptr, nullptr, n, n_pad, 0.f, y,
-                                                      nullptr, nullptr, nullptr);
-  return check_launch ("head_kernel");
+  NetArgs a{};
+  a.params = params;
+  a.wb = (const __nv_bfloat16 *)wbf16;
+  a.X = (const __nv_bfloat16 *)X;
+  a.n = n;
+  a.tiles = n_pad / 128;
+  a.y_out = y;
+  a.err = err;
+  return launch_net<P, false> (a, net_ctas (n_pad), s);
 }
 
 template <int P>
@@ -809,87 +931,23 @@ int train_step_p (const float *params, const void *wbf16, const void *X, const f
                   const float *weight, int n, int n_pad, float *grad, float *loss, void *workspace,
                   int *err, cudaStream_t s)
 {
-  using N = Net<P>;
-  unsigned char *w = (unsigned char *)workspace;
-  const size_t R = (size_t)n_pad;
-  float *Z1 = (float *)w;
-  float *Z2 = Z1 + R * kHid;
-  __nv_bfloat16 *H1 = (__nv_bfloat16 *)(Z2 + R * kHid);
-  __nv_bfloat16 *H2 = H1 + R * kHid;
-  __nv_bfloat16 *dZ2 = H2 + R * kHid;
-  __nv_bfloat16 *dZ1 = dZ2 + R * kHid;
-  __nv_bfloat16 *dZ2T = dZ1 + R * kHid;
-  __nv_bfloat16 *H1T = dZ2T + R * kHid;
-  __nv_bfloat16 *dZ1T = H1T + R * kHid;
-  __nv_bfloat16 *XT = dZ1T + R * kHid;
-  const __nv_bfloat16 *wb = (const __nv_bfloat16 *)wbf16;
-  cudaMemsetAsync (grad, 0, sizeof (float) * N::kParams, s);
-  if (loss) cudaMemsetAsync (loss, 0, sizeof (float), s);
-  int st = forward_layers<P> (params, wb, X, n_pad, Z1, H1, Z2, H2, err, s);
+  NetArgs a{};
+  a.params = params;
+  a.wb = (const __nv_bfloat16 *)wbf16;
+  a.X = (const __nv_bfloat16 *)X;
+  a.target = target;
+  a.weight = weight;
+  a.n = n;
+  a.tiles = n_pad / 128;
+  a.inv_count = 1.f / (float)n;
+  a.partials = (float *)workspace;
+  a.err = err;
+  const int ctas = net_ctas (n_pad);
+  int st = launch_net<P, true> (a, ctas, s);
   if (st) return st;
-  // head, loss, dW3, db3, dZ2, db2
-  head_kernel<P><<<div_up (n_pad, 128), 128, 0, s>>> (params, Z2, target, weight, n, n_pad,
-                                                      1.f / (float)n, nullptr, grad, dZ2, loss);
-  if ((st = check_launch ("head_kernel"))) return st;
-  // dZ1 = (dZ2 W2) x gelu'(Z1): B operand is W2^T
-  GemmArgs b{};
-  b.A = dZ2;
-  b.B = wb + N::kBW2T;
-  b.M = n_pad;
-  b.N = kHid;
-  b.K = kHid;
-  b.k_split = kHid;
-  b.Zin = Z1;
-  b.H = dZ1;
-  b.err = err;
-  if ((st = launch_gemm<EPI_GELU_GRAD> (b, s))) return st;
-  colsum_kernel<<<min (div_up (n_pad, 2), 1024), 256, 0, s>>> (dZ1, n_pad, grad + N::kB1);
-  if ((st = check_launch ("colsum_kernel"))) return st;
-  // transposes for the weight gradients (K = batch)
-  dim3 tb (32, 8);
-  transpose_kernel<<<dim3 (kHid / 32, div_up (n_pad, 32)), tb, 0, s>>> (dZ2, n_pad, kHid, dZ2T);
-  transpose_kernel<<<dim3 (kHid / 32, div_up (n_pad, 32)), tb, 0, s>>> (H1, n_pad, kHid, H1T);
-  transpose_kernel<<<dim3 (kHid / 32, div_up (n_pad, 32)), tb, 0, s>>> (dZ1, n_pad, kHid, dZ1T);
-  transpose_kernel<<<dim3 (div_up (N::kInPad, 32), div_up (n_pad, 32)), tb, 0, s>>> (
-  (const __nv_bfloat16 *)X, n_pad, N::kInPad, XT);
-  if ((st = check_launch ("transpose_kernel"))) return st;
-  const int ksplit = n_pad <= 1024 ? ((n_pad + kKC - 1) / kKC) * kKC : 1024;
-  // dW2 = dZ2^T H1
-  GemmArgs d2{};
-  d2.A = dZ2T;
-  d2.B = H1T;
-  d2.M = kHid;
-  d2.N = kHid;
-  d2.K = n_pad;
-  d2.k_split = ksplit;
-  d2.C = grad + N::kW2;
-  d2.ldc = kHid;
-  d2.ncols = kHid;
-  d2.err = err;
-  if ((st = launch_gemm<EPI_ATOMIC> (d2, s))) return st;
-  GemmArgs d1{};
-  d1.K = n_pad;
-  d1.k_split = ksplit;
-  d1.C = grad + N::kW1;
-  d1.ldc = N::kIn;
-  d1.ncols = N::kIn;
-  d1.err = err;
-  if (N::kInPad <= kGemmN)
-  {
-    // dW1 = dZ1^T X (the first kIn of kInPad columns)
-    d1.A = dZ1T;
-    d1.B = XT;
-    d1.M = kHid;
-    d1.N = N::kInPad;
-    return launch_gemm<EPI_ATOMIC> (d1, s);
-  }
-  // wider inputs: dW1^T = X^T dZ1, rows of the input dimension in 128-row
-  // tiles, stored transposed (the first kIn rows)
-  d1.A = XT;
-  d1.B = dZ1T;
-  d1.M = N::kInPad;
-  d1.N = kHid;
-  return launch_gemm<EPI_ATOMIC_T> (d1, s);
+  constexpr int stride = partial_stride<P> ();
+  reduce_kernel<<<div_up (stride, 128), 256, 0, s>>> (a.partials, ctas, stride, Net<P>::kParams, grad, loss);
+  return check_launch ("reduce_kernel");
 }
 
 template <int P>
@@ -974,9 +1032,8 @@ extern "C" int drb_mlp_features (const drb_mesh *mesh, const int *elem, const fl
                   : features_p<3> (mesh, elem, pts, n, n_pad, X, s);
 }
 
-// Workspace of one training step over n_pad rows (multiple of 128):
-// Z1, Z2 fp32 [n_pad x 128]; H1, H2, dZ2, dZ1 bf16 [n_pad x 128];
-// transposes dZ2T, H1T, dZ1T bf16 [128 x n_pad], XT bf16 [kInPad x n_pad].
+// Workspace of one training step over n_pad rows (multiple of 128): a slot of
+// partial gradients per CTA.
 extern "C" long long drb_mlp_workspace_bytes (int order, int n_pad)
 {
   if (!mlp_order_ok (order) || n_pad < 0) return -1;
@@ -996,9 +1053,9 @@ extern "C" int drb_mlp_forward (int order, const float *params, const void *wbf1
   }
   if (n_pad == 0) return DRB_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  return order == 1 ? forward_p<1> (params, wbf16, X, n, n_pad, y, workspace, err, s)
-         : order == 2 ? forward_p<2> (params, wbf16, X, n, n_pad, y, workspace, err, s)
-                      : forward_p<3> (params, wbf16, X, n, n_pad, y, workspace, err, s);
+  return order == 1 ? forward_p<1> (params, wbf16, X, n, n_pad, y, err, s)
+         : order == 2 ? forward_p<2> (params, wbf16, X, n, n_pad, y, err, s)
+                      : forward_p<3> (params, wbf16, X, n, n_pad, y, err, s);
 }
 
 extern "C" int drb_mlp_train_step (int order, const float *params, const void *wbf16, const void *X,

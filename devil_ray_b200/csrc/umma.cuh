@@ -10,6 +10,13 @@
 // K-adjacent core matrices an instruction reads (128 B) and the
 // stride-dimension byte offset (SBO) the distance between 8-row groups.
 // One kind::f16 instruction consumes K = 16 (two core matrices along K).
+//
+// The same bytes serve as an operand of the transposed matrix (MN-major):
+// the row index r is then K and the column index the operand's row, 8 of
+// them contiguous in a core matrix.  The descriptor's SBO is then the
+// distance between core matrices along the operand's rows (128 B) and its
+// LBO that between the 8-row groups, which are its K ((K / 8) * 128 B), and
+// the instruction descriptor's major bit of that operand is set.
 #pragma once
 
 #include <cstdint>
@@ -46,6 +53,25 @@ DRB_HD constexpr uint32_t idesc_bf16_f32 (int M, int N)
 {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
          ((uint32_t)(M >> 4) << 24);
+}
+
+// The same with A and / or B given MN-major (bits 15 and 16).
+DRB_HD constexpr uint32_t idesc_bf16_f32 (int M, int N, bool a_mn, bool b_mn)
+{
+  return idesc_bf16_f32 (M, N) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16);
+}
+
+// Operand views of a W-wide tile at byte address saddr, from its K offset
+// 16 kk on: rows as the operand's rows (K along the columns), or columns as
+// the operand's rows (K along the tile's rows).
+DRB_D uint64_t desc_rows (uint32_t saddr, int W, int kk)
+{
+  return desc_kmajor (saddr + kk * 256, 128, (uint32_t)(W / 8) * 128);
+}
+DRB_D uint64_t desc_cols (uint32_t saddr, int W, int kk)
+{
+  const uint32_t group = (uint32_t)(W / 8) * 128; // 8 tile rows
+  return desc_kmajor (saddr + kk * 2 * group, group, 128);
 }
 
 // TMEM allocation (one full warp executes these).
@@ -125,6 +151,22 @@ DRB_D void tmem_ld32 (uint32_t taddr, float (&v)[32])
   asm volatile ("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float (r[i]);
+}
+
+// 16 consecutive fp32 columns of this thread's TMEM lane.
+DRB_D void tmem_ld16 (uint32_t taddr, float (&v)[16])
+{
+  uint32_t r[16];
+  asm volatile ("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                  "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                  "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr)
+                : "memory");
+  asm volatile ("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float (r[i]);
 }
 
 } // namespace umma
