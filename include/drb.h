@@ -170,7 +170,8 @@ typedef struct drb_bvh
  * *n_entries; it synchronises the stream.  The caller allocates
  * int32[n_cells + 1], int32[n_entries] and float[8 * n_leaf], sets
  * grid_start, grid_entries and grid_boxes, and calls drb_bvh_grid_build
- * (stream-ordered scratch of about 12 bytes per entry and 32 per leaf).
+ * (stream-ordered scratch of about 4 bytes per entry and per cell; grids with
+ * long lists about 20 bytes per entry).
  * Needs at least two leaves and fewer than 2^31 entries. */
 int drb_bvh_grid_size (drb_bvh *bvh, float cell_scale, long long *n_entries, void *stream);
 int drb_bvh_grid_build (const drb_bvh *bvh, void *stream);

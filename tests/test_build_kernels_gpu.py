@@ -269,3 +269,36 @@ def test_wide_plan_and_emit(cuda, kind, n_elem):
         assert np.array_equal(bits(out.cpu().numpy()), bits(want))
     b.widen()
     assert np.array_equal(bits(b.wide_nodes.cpu().numpy()), bits(want))
+
+
+# scales: lists of a few leaves, of some tens, of about a hundred (more than
+# 64 comparisons an entry: radix passes), and one cell with every leaf
+@pytest.mark.parametrize("n,scale", [(3, 0.4), (5, 1.0), (9, 2.6), (9, 5.0), (4, 1e6)])
+def test_grid_lists_of_every_length(cuda, n, scale):
+    import torch
+    from devil_ray_b200 import api, meshgen
+    m = meshgen.trilinear_distorted_mesh(n, 2, 0.15, seed=11)
+    g = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda)
+    b = g.get_bvh().build_grid(scale)
+    torch.cuda.synchronize()
+    dims, origin, inv = b.grid_geom
+    box = b.grid_boxes.cpu().numpy()
+    lo, hi = box[:, :3], box[:, 4:7]
+
+    def axis(x, d):
+        v = (x - np.float32(origin[d])).astype(np.float32) * np.float32(inv[d])
+        return np.floor(np.clip(v, np.float32(0), np.float32(dims[d] - 1))).astype(np.int64)
+
+    c0 = np.stack([axis(lo[:, d], d) for d in range(3)], 1)
+    span = np.stack([axis(hi[:, d], d) for d in range(3)], 1) - c0 + 1
+    count = span.prod(1)
+    leaf = np.repeat(np.arange(b.n_leaf), count)
+    i = np.arange(leaf.size) - np.repeat(np.cumsum(count) - count, count)
+    s, c = span[leaf], c0[leaf]
+    x, y, z = c[:, 0] + i % s[:, 0], c[:, 1] + i // s[:, 0] % s[:, 1], c[:, 2] + i // (s[:, 0] * s[:, 1])
+    cell = (z * dims[1] + y) * dims[0] + x
+    order = np.lexsort((leaf, cell))
+    n_cells = dims[0] * dims[1] * dims[2]
+    start = np.searchsorted(cell[order], np.arange(n_cells + 1))
+    assert np.array_equal(b.grid_start.cpu().numpy(), start)
+    assert np.array_equal(b.grid_entries.cpu().numpy(), leaf[order])
