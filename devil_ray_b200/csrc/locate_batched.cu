@@ -273,8 +273,13 @@ DRB_D void persistent_body (const LocateParams &lp, const float *__restrict__ pt
     {
       if (pool_next >= pool_end)
       {
-        int base = 0;
-        if (lane == 0) base = atomicAdd (queue_head, chunk);
+        int base = n;
+        if (!queue_head)
+        {
+          // a small batch: one chunk (at most 32 queries) for every warp
+          if (pool_end == 0) base = chunk * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+        }
+        else if (lane == 0) base = atomicAdd (queue_head, chunk);
         base = __shfl_sync (FULL, base, 0);
         if (base >= n)
         {
@@ -541,7 +546,8 @@ struct Staging
 
 template <int P, int W, int S>
 void launch_pw (int mode, dim3 grid, int block, size_t smem, cudaStream_t s, const LocateParams &lp,
-                const GridLists &gl, const float *pts, const int *ord, int n, int chunk, int *head, int *cell, float *ref,
+                const GridLists &gl, const float *pts, const int *ord, int n,
+                int chunk, int *head, int *cell, float *ref,
                 drb_query_stats st, Staging sg)
 {
 #define DRB_LP(K, M, SS) K<P, M, W, SS><<<grid, block, smem, s>>> (lp, pts, ord, n, chunk, head, cell, ref, st.iters, st.candidates, st.nodes, sg.staged, sg.res, gl)
@@ -573,11 +579,19 @@ int traversal_kind (const LocateParams &lp, const GridLists &gl)
   return gl.start ? 2 : lp.wide ? 1 : 0;
 }
 
-int launch_persistent (const drb_mesh *mesh, int mode, dim3 grid, int block, cudaStream_t s,
-                       const LocateParams &lp, const GridLists &gl, const float *pts, const int *ord, int n, int chunk,
+// Shape of a persistent launch: the grid and the queries a warp pops at a time.
+struct LaunchShape
+{
+  int blocks, block, chunk;
+};
+
+int launch_persistent (const drb_mesh *mesh, int mode, const LaunchShape &shape, cudaStream_t s,
+                       const LocateParams &lp, const GridLists &gl, const float *pts, const int *ord, int n,
                        int *head, int *cell, float *ref, drb_query_stats st, Staging sg = Staging ())
 {
   const int order = mesh->order;
+  const dim3 grid ((unsigned)shape.blocks);
+  const int block = shape.block, chunk = shape.chunk;
   const size_t smem = dynamic_smem (order, mode, block);
   const int trav = traversal_kind (lp, gl);
   if (smem > 48 * 1024)
@@ -695,8 +709,8 @@ int check_config (const drb_locate_config &cfg)
 
 // Persistent grid of a launch: the resident blocks of the configured shape
 // on every SM (or cfg.blocks_per_sm of them), no more than the queries fill.
-int persistent_blocks (const drb_mesh *mesh, const drb_bvh *bvh, const drb_locate_config &cfg,
-                       int mode, int n)
+LaunchShape persistent_shape (const drb_mesh *mesh, const drb_bvh *bvh, const drb_locate_config &cfg,
+                              int mode, int n)
 {
   const int per_sm = resident_blocks (mesh, mode, grid_lists (bvh).start ? 2
                                                  : bvh->wide_nodes ? 1 : 0, cfg.block);
@@ -706,7 +720,38 @@ int persistent_blocks (const drb_mesh *mesh, const drb_bvh *bvh, const drb_locat
   const long long blocks_needed = (warps_needed * 32 + cfg.block - 1) / cfg.block;
   if (blocks > blocks_needed) blocks = blocks_needed;
   if (blocks < 1) blocks = 1;
-  return (int)blocks;
+  return { (int)blocks, cfg.block, cfg.chunk };
+}
+
+// Small batches: up to kSmallPerSm queries an SM take one launch of 64-thread
+// blocks without query order or queue; each warp takes one chunk of 1 to 32
+// queries, kSmallWarps warps an SM before the chunks grow.  Such a batch is
+// bound by its slowest query's chain of node loads and Newton steps and by
+// launches: 64 queries a warp ran the sum of two rounds of the slowest lanes,
+// and the order cost five launches.  Measured (us a call, ordered / this):
+// order-2 hexes, grid lists, 1000 queries 55 / 29 (the host's time), 30,000
+// 66 / 38, 100,000 89 / 50, 400,000 136 / 136; order 3, tree, 100,000 139 /
+// 113, 150,000 144 / 138, 250,000 193 / 198, 700,000 308 / 464 (above, the
+// order's coherent warps pay for it); tets, 1000 165 / 47, 100,000 230 / 150.
+// 4 to 32 warps an SM were within 10 % of each other up to 12,000 queries.
+constexpr int kSmallPerSm = 700;
+constexpr int kSmallWarps = 16;
+constexpr int kSmallBlock = 64;
+
+bool small_batch (int n) { return n <= kSmallPerSm * sm_count (); }
+
+LaunchShape small_batch_shape (int n)
+{
+  const int chunk = min (32, div_up (n, kSmallWarps * sm_count ()));
+  return { div_up (div_up (n, chunk), kSmallBlock / 32), kSmallBlock, chunk };
+}
+
+int launch_small (const drb_mesh *mesh, const drb_bvh *bvh, const float *pts, int n,
+                  const drb_newton_opts *opts, int *cell, float *ref, drb_query_stats stats,
+                  cudaStream_t s)
+{
+  return launch_persistent (mesh, kRowsL1, small_batch_shape (n), s, make_params (mesh, bvh, opts),
+                            grid_lists (bvh), pts, nullptr, n, nullptr, cell, ref, stats);
 }
 
 // The persistent kernel over staged query records (head: the queue counter,
@@ -720,13 +765,12 @@ int locate_staged_launch (const drb_mesh *mesh, const drb_bvh *bvh, const float4
   cudaError_t e = cudaMemsetAsync (head, 0, sizeof (int), s);
   if (e != cudaSuccess) return status_from (e);
   const int mode = effective_mode (mesh, cfg.reg_elements);
-  const int blocks = persistent_blocks (mesh, bvh, cfg, mode, n);
+  const LaunchShape shape = persistent_shape (mesh, bvh, cfg, mode, n);
   const LocateParams lp = make_params (mesh, bvh, opts);
   Staging sg;
   sg.staged = staged;
   sg.res = res;
-  return launch_persistent (mesh, mode, dim3 ((unsigned)blocks), cfg.block, s, lp, grid_lists (bvh),
-                            nullptr, nullptr, n, cfg.chunk, head, cell, ref, stats, sg);
+  return launch_persistent (mesh, mode, shape, s, lp, grid_lists (bvh), nullptr, nullptr, n, head, cell, ref, stats, sg);
 }
 
 // Sorted, staged batch over caller buffers: stage the queries in Morton-cell
@@ -761,6 +805,8 @@ int locate_batched_impl (const drb_mesh *mesh, const drb_bvh *bvh, const float *
   if (n == 0) return DRB_OK;
   const drb_locate_config cfg = cfg_in ? *cfg_in : default_config (mesh->order);
   if ((st = check_config (cfg))) return st;
+  if (!order_in && small_batch (n))
+    return launch_small (mesh, bvh, pts, n, opts, cell, ref, stats, s);
   Scratch scr (s);
   int *head = scr.alloc<int> (1);
   if (!order_in && cfg.sort_queries >= kSortStaged)
@@ -794,11 +840,10 @@ int locate_batched_impl (const drb_mesh *mesh, const drb_bvh *bvh, const float *
   if (scr.err != cudaSuccess) return status_from (scr.err);
   cudaMemsetAsync (head, 0, sizeof (int), s);
   const int mode = effective_mode (mesh, cfg.reg_elements);
-  const int blocks = persistent_blocks (mesh, bvh, cfg, mode, n);
+  const LaunchShape shape = persistent_shape (mesh, bvh, cfg, mode, n);
   const LocateParams lp = make_params (mesh, bvh, opts);
-  return launch_persistent (mesh, mode, dim3 ((unsigned)blocks), cfg.block, s, lp, grid_lists (bvh),
-                            pts, ord, n,
-                            cfg.chunk, head, cell, ref, stats);
+  return launch_persistent (mesh, mode, shape, s, lp, grid_lists (bvh), pts, ord, n, head, cell, ref,
+                            stats);
 }
 
 // Same as locate_batched_impl with sorting (queries read through the index
@@ -813,6 +858,7 @@ int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pt
   if (n == 0) return DRB_OK;
   const drb_locate_config cfg = cfg_in ? *cfg_in : default_config (mesh->order);
   if ((st = check_config (cfg))) return st;
+  if (small_batch (n)) return launch_small (mesh, bvh, pts, n, opts, cell, ref, stats, s);
   const int *ord = nullptr;
   if (cfg.sort_queries)
   {
@@ -823,11 +869,10 @@ int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pt
   cudaError_t e = cudaMemsetAsync (ws.head, 0, sizeof (int), s);
   if (e != cudaSuccess) return status_from (e);
   const int mode = effective_mode (mesh, cfg.reg_elements);
-  const int blocks = persistent_blocks (mesh, bvh, cfg, mode, n);
+  const LaunchShape shape = persistent_shape (mesh, bvh, cfg, mode, n);
   const LocateParams lp = make_params (mesh, bvh, opts);
-  return launch_persistent (mesh, mode, dim3 ((unsigned)blocks), cfg.block, s, lp, grid_lists (bvh),
-                            pts, ord, n,
-                            cfg.chunk, ws.head, cell, ref, stats);
+  return launch_persistent (mesh, mode, shape, s, lp, grid_lists (bvh), pts, ord, n, ws.head, cell,
+                            ref, stats);
 }
 
 } // namespace drb
