@@ -701,13 +701,97 @@ DRB_D void finish_ray (RayMarch &s, float4 *__restrict__ fb_color, float *__rest
   s.i = -1;
 }
 
+// One sample into its ray: blend a located one, and apply the segment and ray
+// termination rules of integrate_partials (a segment ends at the first sample
+// not located, at the ray's far distance or when its alpha reaches 0.95; the
+// ray ends after 5 segments, at far, or when alpha exceeds 0.95).  Returns
+// true when the ray is done.
+DRB_D bool take_sample (RayMarch &s, bool found, const float4 &sc, float sample_dist,
+                        VolumePartial *__restrict__ partials)
+{
+  constexpr int kMaxSegments = 5; // volume.cpp:110
+  bool done = false;
+  if (found)
+  {
+    if (!s.in_seg)
+    {
+      s.in_seg = true;
+      s.seg_depth = s.distance;
+      s.color = make_float4 (0.f, 0.f, 0.f, 0.f);
+    }
+    ++s.n_samples;
+    blend (s.color, sc);
+    s.distance += sample_dist;
+    if (!(s.distance < s.ray.far_t) || !(s.color.w < 0.95f))
+    {
+      const float alpha = s.color.w;
+      end_segment (s, partials);
+      done = !(s.distance < s.ray.far_t) || alpha > 0.95f || s.segment == kMaxSegments;
+    }
+  }
+  else
+  {
+    if (s.in_seg)
+    {
+      end_segment (s, partials);
+      done = s.segment == kMaxSegments;
+    }
+    s.distance += sample_dist;
+    if (!(s.distance < s.ray.far_t)) done = true;
+  }
+  return done;
+}
+
+// The march's state before a ray's first sample; false when the ray has none.
+DRB_D bool start_ray (const VolumeParams &vp, RayMarch &s)
+{
+  bool live = true;
+  if (vp.cull)
+  {
+    // mark_active + calc_ray_start (ray.cpp:117-241) on the raw ray
+    float t0, t1;
+    live = slab (s.ray, vp.box, t0, t1);
+    s.ray.near_t = t0;
+    s.ray.far_t = t1;
+  }
+  s.distance = s.ray.near_t + vp.sample_dist;
+  s.segment = 0;
+  s.in_seg = false;
+  s.color = make_float4 (0.f, 0.f, 0.f, 0.f);
+  s.pixel = make_float4 (0.f, 0.f, 0.f, 0.f);
+  s.first_depth = INFINITY;
+  s.seg_depth = 0.f;
+  s.prev_el = -1;
+  s.prev_ref[0] = s.prev_ref[1] = s.prev_ref[2] = 0.5f;
+  s.prev2_ok = false;
+  s.prev2_ref[0] = s.prev2_ref[1] = s.prev2_ref[2] = 0.5f;
+  s.n_samples = s.iters = s.cands = s.nodes = 0;
+  return live && s.distance < s.ray.far_t;
+}
+
+// A located sample becomes the start of the next one's prediction.
+DRB_D void keep_sample (const VolumeParams &vp, RayMarch &s, int el, const float (&ref)[3])
+{
+  if (el < 0)
+  {
+    s.prev_el = -1;
+    s.prev2_ok = false;
+    return;
+  }
+  s.prev2_ok = vp.quadratic_predictor && el == s.prev_el;
+  s.prev_el = el;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+  {
+    s.prev2_ref[d] = s.prev_ref[d];
+    s.prev_ref[d] = ref[d];
+  }
+}
+
 // Persistent march: warps pop chunks of rays from a global queue and keep
 // every lane on a ray (ballot refill, as the batched locate does with
 // queries).  Each loop iteration advances every busy lane by one sample:
-// locate (coherent or full), shade, blend, and the segment and ray
-// termination rules of integrate_partials: a segment ends at the first
-// sample not located, at the ray's far distance or when its alpha reaches
-// 0.95; the ray ends after 5 segments, at far, or when alpha exceeds 0.95.
+// locate (coherent or full), shade, take_sample.
 // Partials go to slot 5 i + segment of ray i and the framebuffer pixel gets
 // their front-to-back composite, so the processing order changes nothing.
 template <int P, bool WIDE, int S>
@@ -717,7 +801,6 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
                float *__restrict__ fb_depth, int *__restrict__ ray_samples,
                int *__restrict__ ray_iters, int *__restrict__ ray_cands)
 {
-  constexpr int kMaxSegments = 5; // volume.cpp:110
   constexpr int kChunk = 32;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -753,32 +836,11 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
       {
         s.i = pool_next + rank;
         s.ray = rays[s.i];
-        bool live = true;
-        if (vp.cull)
-        {
-          // mark_active + calc_ray_start (ray.cpp:117-241) on the raw ray
-          float t0, t1;
-          live = slab (s.ray, vp.box, t0, t1);
-          s.ray.near_t = t0;
-          s.ray.far_t = t1;
-        }
-        s.distance = s.ray.near_t + vp.sample_dist;
-        s.segment = 0;
-        s.in_seg = false;
-        s.color = make_float4 (0.f, 0.f, 0.f, 0.f);
-        s.pixel = make_float4 (0.f, 0.f, 0.f, 0.f);
-        s.first_depth = INFINITY;
-        s.seg_depth = 0.f;
-        s.prev_el = -1;
-        s.prev_ref[0] = s.prev_ref[1] = s.prev_ref[2] = 0.5f;
-        s.prev2_ok = false;
-        s.prev2_ref[0] = s.prev2_ref[1] = s.prev2_ref[2] = 0.5f;
-        s.n_samples = s.iters = s.cands = s.nodes = 0;
+        const bool live = start_ray (vp, s);
         step[0] = s.ray.dir.x * vp.sample_dist;
         step[1] = s.ray.dir.y * vp.sample_dist;
         step[2] = s.ray.dir.z * vp.sample_dist;
-        if (!live || !(s.distance < s.ray.far_t))
-          finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+        if (!live) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
       }
       pool_next += min (__popc (need), avail);
       need = __ballot_sync (FULL, s.i < 0);
@@ -793,47 +855,130 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
     float ref[3];
     const int el = locate_sample<P, WIDE, S> (vp, pt, step, s.prev_el, s.prev_ref, s.prev2_ok,
                                               s.prev2_ref, lu, ref, s.iters, s.cands, s.nodes);
-    bool done = false;
-    if (el >= 0)
+    float4 sc = make_float4 (0.f, 0.f, 0.f, 0.f);
+    if (el >= 0) sc = shade_sample<P, S> (vp, el, ref, s.ray, lu, pt);
+    keep_sample (vp, s, el, ref);
+    if (take_sample (s, el >= 0, sc, vp.sample_dist, partials))
+      finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+  }
+}
+
+// The plain march of few rays: a group of G lanes (4 to 32, a power of two)
+// takes G consecutive samples of one ray at once.  Every lane locates and
+// shades its own sample; then the group's samples are blended in ray order,
+// each lane repeating the same steps on values passed by shuffle, so the
+// result is the one-lane march's bit for bit (a plain sample does not depend
+// on the one before it, and the distances are the same repeated sums).
+// Samples behind the one that ends the ray are thrown away.  Bound, like the
+// one-lane march, by the chains of node loads and Newton steps; the lanes give
+// the SMs enough of them.  256^2 pixels, 500 samples, 8^3 order-2 hexes: 4.32
+// -> 2.06 ms a frame.
+template <int P, bool WIDE, int S>
+__global__ void __launch_bounds__ (128)
+volume_group_kernel (VolumeParams vp, int G, const Ray *__restrict__ rays, int n_rays,
+                     int *__restrict__ queue, VolumePartial *__restrict__ partials,
+                     float4 *__restrict__ fb_color, float *__restrict__ fb_depth,
+                     int *__restrict__ ray_samples, int *__restrict__ ray_iters,
+                     int *__restrict__ ray_cands)
+{
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int g = lane & (G - 1);
+  const int lead = lane - g;                 // the group's first lane
+  RayMarch s;
+  s.i = -1;
+  bool exhausted = false; // warp-uniform
+  while (true)
+  {
+    // ---- give idle groups the next rays ----
+    unsigned need = __ballot_sync (FULL, s.i < 0 && g == 0);
+    while (need != 0u && !exhausted)
     {
-      if (!s.in_seg)
+      int base = 0;
+      if (lane == 0) base = atomicAdd (queue, __popc (need));
+      base = __shfl_sync (FULL, base, 0);
+      exhausted = base + __popc (need) >= n_rays;
+      const int i = base + __popc (need & ((1u << lead) - 1u));
+      if (s.i < 0 && i < n_rays)
       {
-        s.in_seg = true;
-        s.seg_depth = s.distance;
-        s.color = make_float4 (0.f, 0.f, 0.f, 0.f);
+        s.i = i;
+        s.ray = rays[i];
+        if (!start_ray (vp, s))
+        {
+          if (g == 0) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+          s.i = -1;
+        }
       }
-      ++s.n_samples;
-      const float4 sc = shade_sample<P, S> (vp, el, ref, s.ray, lu, pt);
-      blend (s.color, sc);
-      s.prev2_ok = vp.quadratic_predictor && el == s.prev_el;
-      s.prev2_ref[0] = s.prev_ref[0];
-      s.prev2_ref[1] = s.prev_ref[1];
-      s.prev2_ref[2] = s.prev_ref[2];
-      s.prev_el = el;
-      s.prev_ref[0] = ref[0];
-      s.prev_ref[1] = ref[1];
-      s.prev_ref[2] = ref[2];
-      s.distance += vp.sample_dist;
-      if (!(s.distance < s.ray.far_t) || !(s.color.w < 0.95f))
+      need = __ballot_sync (FULL, s.i < 0 && g == 0);
+    }
+    if (__ballot_sync (FULL, s.i >= 0) == 0u) break;
+
+    // ---- this lane's sample: the group's next distance plus g steps ----
+    float dist = s.distance, t = s.distance;
+    for (int k = 0; k < G; ++k)
+    {
+      if (k == g) dist = t;
+      t += vp.sample_dist;
+    }
+    int el = -1, iters = 0, cands = 0;
+    float4 sc = make_float4 (0.f, 0.f, 0.f, 0.f);
+    if (s.i >= 0 && dist < s.ray.far_t)
+    {
+      const float pt[3] = { s.ray.orig.x + dist * s.ray.dir.x, s.ray.orig.y + dist * s.ray.dir.y,
+                            s.ray.orig.z + dist * s.ray.dir.z };
+      float ref[3];
+      LU3 lu;
+      el = locate_sample<P, WIDE, S> (vp, pt, pt, -1, pt, false, pt, lu, ref, iters, cands, s.nodes);
+      if (el >= 0) sc = shade_sample<P, S> (vp, el, ref, s.ray, lu, pt);
+    }
+    __syncwarp ();
+
+    // ---- blend the group's samples in ray order ----
+    bool busy = s.i >= 0;
+    const unsigned hit = __ballot_sync (FULL, el >= 0) >> lead;
+    int used = 0; // samples taken
+    for (int k = 0; k < G; ++k)
+    {
+      float4 c;
+      c.x = __shfl_sync (FULL, sc.x, lead + k);
+      c.y = __shfl_sync (FULL, sc.y, lead + k);
+      c.z = __shfl_sync (FULL, sc.z, lead + k);
+      c.w = __shfl_sync (FULL, sc.w, lead + k);
+      if (busy)
       {
-        const float alpha = s.color.w;
-        end_segment (s, partials);
-        done = !(s.distance < s.ray.far_t) || alpha > 0.95f || s.segment == kMaxSegments;
+        ++used;
+        busy = !take_sample (s, (hit >> k) & 1u, c, vp.sample_dist, g == 0 ? partials : nullptr);
+      }
+      if (__ballot_sync (FULL, busy) == 0u) break;
+    }
+    if (g < used)
+    {
+      s.iters += iters;
+      s.cands += cands;
+    }
+    const bool done = s.i >= 0 && !busy;
+    if (ray_iters || ray_cands)
+    {
+      if (__ballot_sync (FULL, done))
+      {
+        int it = s.iters, ca = s.cands;
+        for (int o = G >> 1; o; o >>= 1)
+        {
+          it += __shfl_xor_sync (FULL, it, o);
+          ca += __shfl_xor_sync (FULL, ca, o);
+        }
+        if (done)
+        {
+          s.iters = it;
+          s.cands = ca;
+        }
       }
     }
-    else
+    if (done)
     {
-      s.prev_el = -1;
-      s.prev2_ok = false;
-      if (s.in_seg)
-      {
-        end_segment (s, partials);
-        done = s.segment == kMaxSegments;
-      }
-      s.distance += vp.sample_dist;
-      if (!(s.distance < s.ray.far_t)) done = true;
+      if (g == 0) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+      s.i = -1;
     }
-    if (done) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
   }
 }
 
@@ -934,18 +1079,47 @@ __global__ void fb_background_kernel (float4 *c, int n, float4 bg)
   }
 }
 
+// Lanes per ray of the plain march.  One lane per ray wins as long as the rays
+// fill the SMs (512 threads each at 128 registers): its warps stay on
+// neighbouring rays at one depth, and no sample is thrown away.  With fewer
+// rays than half of that, the march is one chain of locates per lane and the
+// SMs idle, so a ray gets as many lanes as make about six waves of them, up to
+// 32.  Measured (us a frame, 1 lane / 8 / 16 / 32 lanes): 256^2 pixels, 500
+// samples, 8^3 order-2 hexes 4197 / 2217 / 2066 / 2358; 128^2, 300 samples,
+// 20^3 order 3 3163 / 1349 / 1078 / 998; 300^2, 200 samples, 10^3 x 6 order-2
+// tets 8629 / 7048 / 7005 / 7942; 512^2 of the order-3 hexes 6358 / 9177 / 9922
+// / 11461.  The coherent march keeps one lane: predicting several samples ahead
+// was up to twice as fast on small frames, but samples on shared faces then
+// fell to other elements than before.
+int group_lanes (const VolumeParams &vp, int n)
+{
+  const int lanes = 512 * sm_count ();
+  if (vp.coherent || n > lanes / 2) return 1;
+  int G = 4;
+  while (2 * G <= min (32, 6 * lanes / n)) G *= 2;
+  return G;
+}
+
 template <int P, bool WIDE, int S>
 int launch_volume_w (const VolumeParams &vp, const Ray *rays, int n, int *queue,
                      VolumePartial *partials, float4 *fb, float *depth, const drb_ray_stats &st,
                      cudaStream_t s)
 {
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, volume_kernel<P, WIDE, S>, 128, 0);
+  const int G = group_lanes (vp, n);
+  if (G > 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, volume_group_kernel<P, WIDE, S>, 128, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, volume_kernel<P, WIDE, S>, 128, 0);
   if (nb < 1) nb = 1;
   long long blocks = (long long)nb * sm_count ();
-  const long long need = ((long long)n + 127) / 128;
+  const long long need = ((long long)n * G + 127) / 128;
   if (blocks > need) blocks = need;
   if (blocks < 1) blocks = 1;
+  if (G > 1)
+  {
+    volume_group_kernel<P, WIDE, S><<<(unsigned)blocks, 128, 0, s>>> (
+        vp, G, rays, n, queue, partials, fb, depth, st.samples, st.iters, st.candidates);
+    return check_launch ("volume_group_kernel");
+  }
   volume_kernel<P, WIDE, S><<<(unsigned)blocks, 128, 0, s>>> (vp, rays, n, queue, partials, fb, depth,
                                                               st.samples, st.iters, st.candidates);
   return check_launch ("volume_kernel");

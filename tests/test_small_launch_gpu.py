@@ -1,9 +1,9 @@
-"""The launch shape for few queries against the one for many: the same queries
-give the same bits."""
+"""The launch shapes for few queries and few rays against the ones for many:
+the same queries and rays give the same bits."""
 import pytest
 
 from devil_ray_b200 import _lib as L
-from devil_ray_b200 import api, meshgen
+from devil_ray_b200 import api, meshgen, render
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +30,49 @@ def test_small_batch_equals_ordered(cuda, kind, p, lists, count):
     order = torch.arange(count, dtype=torch.int32, device=cuda).flip(0).contiguous()
     for a, b in zip(loc.locate(q, stats=True), loc.locate(q, order=order, stats=True)):
         assert torch.equal(a, b)
+
+
+# rays: 32 lanes each, 8 or so, 4, and (above half the SMs' lanes) one
+@pytest.mark.parametrize("kind,p,lit", [("hex", 1, True), ("hex", 2, False), ("hex", 3, True),
+                                        ("tet", 2, True)])
+def test_few_rays_equal_many(cuda, kind, p, lit):
+    import torch
+    m, shape = _mesh(kind, 4, p)
+    mesh = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda, shape=shape)
+    values = torch.sin(7.0 * torch.as_tensor(m.xyz, device=cuda)).sum(1).float()
+    field = render.UnstructuredField(m.ctrl_idx, values, m.order, device=cuda, shape=shape)
+    c = meshgen.CAMERA
+    camera = render.Camera(512, 512, c["pos"], c["look_at"], c["up"], c["fov"])
+    light = [render.PointLight.default(camera)]
+    active = render.cull_rays(camera.create_rays(cuda), mesh.bounds())
+    assert active.shape[0] > 37888
+    for opacity in (0.02, 0.9):
+        vol = render.Volume(mesh, field)
+        table = render.ColorTable()
+        table.add_point(0.0, (0.1, 0.2, 0.9))
+        table.add_point(1.0, (0.9, 0.4, 0.1))
+        table.add_alpha(0.0, 0.0)
+        table.add_alpha(1.0, opacity)
+        vol.color_map().color_table(table)
+        vol.samples(37)
+        vol.use_lighting(lit)
+        whole, stats = vol.render(camera, light, active=active, stats=True)
+        colors, depths = whole.colors.clone(), whole.depths.clone()
+        parts = torch.zeros_like(colors)
+        first, got = 0, []
+        fb = render.Framebuffer(512, 512, cuda)
+        seen = torch.full_like(depths, float("inf"))
+        for size in (1, 100, 2500, 12000, 20000, active.shape[0]):
+            some = active[first:min(first + size, first + 30000)].contiguous()
+            if some.shape[0] == 0:
+                break
+            _, st = vol.render(camera, light, fb=fb, active=some, stats=True)
+            hit = torch.isfinite(fb.depths)
+            parts[hit], seen[hit] = fb.colors[hit], fb.depths[hit]
+            got.append([s[:some.shape[0]].clone() for s in st])
+            first += some.shape[0]
+        for k in range(3):
+            assert torch.equal(torch.cat([g[k] for g in got]), stats[k][:first])
+        done = torch.isfinite(seen)
+        assert done.sum() > 1000
+        assert torch.equal(parts[done], colors[done]) and torch.equal(seen[done], depths[done])
