@@ -237,8 +237,14 @@ struct LU3
   int perm[3];
   bool valid;
 
-  DRB_D void factor (const float (&m)[3][3])
+  // Factors m and solves m x = b on the way: b's rows move and are eliminated
+  // with the matrix's, so the permutation is only kept where lu is used again.
+  // The steps are those of a factorisation and solve (), which multiplies by
+  // the reciprocals of the pivots that stand on the diagonal: three divisions
+  // a step of Newton's iteration instead of six.
+  DRB_D void factor_solve (const float (&m)[3][3], const float (&b)[3], float (&x)[3])
   {
+    float y[3] = { b[0], b[1], b[2] };
 #pragma unroll
     for (int r = 0; r < 3; ++r)
     {
@@ -281,17 +287,26 @@ struct LU3
             const int tp = perm[r];
             perm[r] = perm[t];
             perm[t] = tp;
+            const float ty = y[r];
+            y[r] = y[t];
+            y[t] = ty;
           }
         }
       }
       // upper-triangle elements (MatrixLUPFactorFindUpperTriangleElements)
+      const float rp = 1.f / a[t][t];
 #pragma unroll
-      for (int c = t + 1; c < 3; ++c) a[t][c] = a[t][c] / a[t][t];
+      for (int c = t + 1; c < 3; ++c) a[t][c] *= rp;
 #pragma unroll
       for (int r = t + 1; r < 3; ++r)
 #pragma unroll
         for (int c = t + 1; c < 3; ++c) a[r][c] -= a[r][t] * a[t][c];
+      a[t][t] = rp;
+      y[t] *= rp;
+#pragma unroll
+      for (int r = t + 1; r < 3; ++r) y[r] -= a[r][t] * y[t];
     }
+    back_substitute (y, x);
   }
 
   DRB_D void solve (const float (&b)[3], float (&x)[3]) const
@@ -304,8 +319,13 @@ struct LU3
       y[r] = pr == 0 ? b[0] : (pr == 1 ? b[1] : b[2]);
 #pragma unroll
       for (int c = 0; c < r; ++c) y[r] -= a[r][c] * y[c];
-      y[r] = y[r] / a[r][r];
+      y[r] *= a[r][r];
     }
+    back_substitute (y, x);
+  }
+
+  DRB_D void back_substitute (const float (&y)[3], float (&x)[3]) const
+  {
 #pragma unroll
     for (int r = 2; r >= 0; --r)
     {

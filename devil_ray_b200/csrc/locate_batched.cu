@@ -230,7 +230,9 @@ template <int P> constexpr size_t smem_rows_bytes_per_warp ()
 // go to res[pos] as (cell as int bits, reference point), contiguous, for a
 // separate pass to put back.  Statistics always go to the input index.
 // TRAV: 0 binary tree, 1 4-wide tree, 2 grid candidate lists.
-template <int P, int MODE, int TRAV, int S>
+// SMALL: no queue; each warp takes the one chunk (at most 32 queries) that its
+// number in the grid says.
+template <int P, int MODE, int TRAV, int S, bool SMALL>
 DRB_D void persistent_body (const LocateParams &lp, const float *__restrict__ pts,
                                             const int *__restrict__ order, int n, int chunk,
                                             int *__restrict__ queue_head, int *__restrict__ cell,
@@ -274,13 +276,12 @@ DRB_D void persistent_body (const LocateParams &lp, const float *__restrict__ pt
       if (pool_next >= pool_end)
       {
         int base = n;
-        if (!queue_head)
+        if (!SMALL)
         {
-          // a small batch: one chunk (at most 32 queries) for every warp
-          if (pool_end == 0) base = chunk * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+          if (lane == 0) base = atomicAdd (queue_head, chunk);
+          base = __shfl_sync (FULL, base, 0);
         }
-        else if (lane == 0) base = atomicAdd (queue_head, chunk);
-        base = __shfl_sync (FULL, base, 0);
+        else if (pool_end == 0) base = chunk * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
         if (base >= n)
         {
           exhausted = true;
@@ -468,23 +469,33 @@ DRB_D void persistent_body (const LocateParams &lp, const float *__restrict__ pt
 template <int P, int MODE, int TRAV, int S = kTensor>
 __global__ void locate_persistent_kernel (DRB_PERSISTENT_ARGS)
 {
-  persistent_body<P, MODE, TRAV, S> (lp, pts, order, n, chunk, queue_head, cell, ref, it_out, ca_out,
+  persistent_body<P, MODE, TRAV, S, false> (lp, pts, order, n, chunk, queue_head, cell, ref, it_out, ca_out,
                                      nd_out, staged, res, gl);
 }
-// The grid scan with L1 rows at orders 1-2, held to 80 registers (the
-// compiler's choice of 89 at order 2 costs a quarter of the resident warps;
-// measured 9 % faster at 80, slower at 72, where it spills).
+// Hexes with L1 rows, and every kind's grid scan at orders 1-2, held to the
+// registers that still give a full set of resident warps.  Left alone the
+// compiler's choice moves with small changes of the code: order 2 over grid
+// lists 89 registers (9 % slower than at 80, and 72 spills), order 3 109 to 115
+// (1M queries over the tree 414 us against 375 at 96, over grid lists 315
+// against 284); order 2 over the tree spills at 72 (545 us against 529).
+template <int P> constexpr int max_regs () { return P == 3 ? 96 : 80; }
 template <int P, int MODE, int TRAV, int S = kTensor>
-__global__ void __maxnreg__ (80) locate_persistent_kernel_r80 (DRB_PERSISTENT_ARGS)
+__global__ void __maxnreg__ (max_regs<P> ()) locate_persistent_kernel_capped (DRB_PERSISTENT_ARGS)
 {
-  persistent_body<P, MODE, TRAV, S> (lp, pts, order, n, chunk, queue_head, cell, ref, it_out, ca_out,
+  persistent_body<P, MODE, TRAV, S, false> (lp, pts, order, n, chunk, queue_head, cell, ref, it_out, ca_out,
                                      nd_out, staged, res, gl);
+}
+template <int P, int TRAV, int S = kTensor>
+__global__ void locate_small_kernel (DRB_PERSISTENT_ARGS)
+{
+  persistent_body<P, kRowsL1, TRAV, S, true> (lp, pts, order, n, chunk, queue_head, cell, ref, it_out,
+                                              ca_out, nd_out, staged, res, gl);
 }
 #undef DRB_PERSISTENT_ARGS
 
-template <int P, int MODE, int TRAV> constexpr bool capped_kernel ()
+template <int P, int MODE, int TRAV, int S> constexpr bool capped_kernel ()
 {
-  return TRAV == 2 && MODE == kRowsL1 && P <= 2;
+  return MODE == kRowsL1 && (S == kTensor || (P <= 2 && TRAV == 2));
 }
 
 // Tets run the L1 and register row modes (shared rows are tensor-only).
@@ -492,8 +503,8 @@ template <int P, int W, int S> const void *persistent_fn_pw (int mode)
 {
   if (S == kTensor && mode == kRowsShared) return (const void *)locate_persistent_kernel<P, kRowsShared, W>;
   if (mode == kRowsReg && P <= 2) return (const void *)locate_persistent_kernel<P, kRowsReg, W, S>;
-  if constexpr (capped_kernel<P, kRowsL1, W> ())
-    return (const void *)locate_persistent_kernel_r80<P, kRowsL1, W, S>;
+  if constexpr (capped_kernel<P, kRowsL1, W, S> ())
+    return (const void *)locate_persistent_kernel_capped<P, kRowsL1, W, S>;
   else
     return (const void *)locate_persistent_kernel<P, kRowsL1, W, S>;
 }
@@ -551,9 +562,11 @@ void launch_pw (int mode, dim3 grid, int block, size_t smem, cudaStream_t s, con
                 drb_query_stats st, Staging sg)
 {
 #define DRB_LP(K, M, SS) K<P, M, W, SS><<<grid, block, smem, s>>> (lp, pts, ord, n, chunk, head, cell, ref, st.iters, st.candidates, st.nodes, sg.staged, sg.res, gl)
-  if (S == kTensor && mode == kRowsShared) DRB_LP (locate_persistent_kernel, kRowsShared, kTensor);
+  if (!head)
+    locate_small_kernel<P, W, S><<<grid, block, smem, s>>> (lp, pts, ord, n, chunk, head, cell, ref, st.iters, st.candidates, st.nodes, sg.staged, sg.res, gl);
+  else if (S == kTensor && mode == kRowsShared) DRB_LP (locate_persistent_kernel, kRowsShared, kTensor);
   else if (mode == kRowsReg && P <= 2) DRB_LP (locate_persistent_kernel, P <= 2 ? kRowsReg : kRowsL1, S);
-  else if constexpr (capped_kernel<P, kRowsL1, W> ()) DRB_LP (locate_persistent_kernel_r80, kRowsL1, S);
+  else if constexpr (capped_kernel<P, kRowsL1, W, S> ()) DRB_LP (locate_persistent_kernel_capped, kRowsL1, S);
   else DRB_LP (locate_persistent_kernel, kRowsL1, S);
 #undef DRB_LP
 }
@@ -579,7 +592,8 @@ int traversal_kind (const LocateParams &lp, const GridLists &gl)
   return gl.start ? 2 : lp.wide ? 1 : 0;
 }
 
-// Shape of a persistent launch: the grid and the queries a warp pops at a time.
+// Shape of a persistent launch: the grid and the queries a warp pops at a time
+// (a launch without a queue head is a small batch's).
 struct LaunchShape
 {
   int blocks, block, chunk;

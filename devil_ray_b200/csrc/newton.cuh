@@ -62,8 +62,7 @@ DRB_D void hex_step (const CP &cp, const float (&target)[3], float (&x)[3], LU3 
     J[r][1] = Jv[r];
     J[r][2] = Jw[r];
   }
-  lu.factor (J);
-  lu.solve (dy, dx);
+  lu.factor_solve (J, dy, dx);
 #pragma unroll
   for (int d = 0; d < 3; ++d) x[d] += dx[d];
 }
@@ -124,8 +123,7 @@ DRB_D void quad_step (const CP &cp, const float (&target)[3], float (&x)[3], LU3
     J[r][1] = Jv[r];
     J[r][2] = (r == 2) ? 1.f : 0.f;
   }
-  lu.factor (J);
-  lu.solve (dy, dx);
+  lu.factor_solve (J, dy, dx);
   x[0] += dx[0];
   x[1] += dx[1];
 }

@@ -342,8 +342,7 @@ DRB_D bool face_newton (const CP &cp, const Ray &ray, float (&x)[2], float &t, f
       J[r][2] = -d[r];
     }
     LU3 lu;
-    lu.factor (J);
-    lu.solve (dy, dx);
+    lu.factor_solve (J, dy, dx);
     x[0] += dx[0];
     x[1] += dx[1];
     t = dx[2];
