@@ -334,6 +334,28 @@ struct LU3
       for (int c = r + 1; c < 3; ++c) x[r] -= a[r][c] * x[c];
     }
   }
+
+  // x with the transposed matrix: U^T z = b, L^T w = z, x = P^T w.
+  DRB_D void solve_transposed (const float (&b)[3], float (&x)[3]) const
+  {
+    float w[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+    {
+      w[r] = b[r];
+#pragma unroll
+      for (int c = 0; c < r; ++c) w[r] -= a[c][r] * w[c];
+    }
+#pragma unroll
+    for (int r = 2; r >= 0; --r)
+    {
+#pragma unroll
+      for (int c = r + 1; c < 3; ++c) w[r] -= a[c][r] * w[c];
+      w[r] *= a[r][r];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) x[i] = perm[0] == i ? w[0] : (perm[1] == i ? w[1] : w[2]);
+  }
 };
 
 } // namespace drb

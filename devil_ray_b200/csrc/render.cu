@@ -406,36 +406,19 @@ DRB_D float4 shade_sample (const VolumeParams &vp, int el, const float (&r)[3], 
   if (!vp.use_lighting) return c;
   float4 acc = make_float4 (0.f, 0.f, 0.f, 0.f);
   if (!(c.w > 0.01f)) return acc;
-  // matrix_inverse via LUP (matrix.hpp:430-456); gradient = gref * J^-1
-  float inv[3][3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-  {
-    float e[3] = { 0.f, 0.f, 0.f };
-    e[c] = 1.f;
-    float col[3];
-    lu.solve (e, col);
-#pragma unroll
-    for (int rr = 0; rr < 3; ++rr) inv[rr][c] = col[rr];
-  }
-  Vec3 g;
-  g.x = gref[0] * inv[0][0] + gref[1] * inv[1][0] + gref[2] * inv[2][0];
-  g.y = gref[0] * inv[0][1] + gref[1] * inv[1][1] + gref[2] * inv[2][1];
-  g.z = gref[0] * inv[0][2] + gref[1] * inv[1][2] + gref[2] * inv[2][2];
-  {
-    const float m = sqrtf (dot (g, g));
-    g = make3 (g.x / m, g.y / m, g.z / m);
-  }
+  // gradient = gref * J^-1 (the reference multiplies by the inverse,
+  // matrix.hpp:430-456): one solve with the transposed factors
+  float gw[3];
+  lu.solve_transposed (gref, gw);
+  Vec3 g = make3 (gw[0], gw[1], gw[2]);
+  g = (1.f / sqrtf (dot (g, g))) * g;
   const Vec3 view = make3 (-ray.dir.x, -ray.dir.y, -ray.dir.z);
   const Vec3 wp = make3 (wpos[0], wpos[1], wpos[2]);
   for (int l = 0; l < vp.n_lights; ++l)
   {
     const PointLight L = vp.lights[l];
     Vec3 ld = make3 (L.pos[0] - wp.x, L.pos[1] - wp.y, L.pos[2] - wp.z);
-    {
-      const float m = sqrtf (dot (ld, ld));
-      ld = make3 (ld.x / m, ld.y / m, ld.z / m);
-    }
+    ld = (1.f / sqrtf (dot (ld, ld))) * ld;
     if (dot (ld, g) < 0.f) g = make3 (-g.x, -g.y, -g.z);
     const float diffuse = clampf (dot (ld, g), 0.f, 1.f);
     float sc[4] = { L.amb[0] * c.x, L.amb[1] * c.y, L.amb[2] * c.z, c.w };
@@ -443,10 +426,7 @@ DRB_D float4 shade_sample (const VolumeParams &vp, int el, const float (&r)[3], 
 #pragma unroll
     for (int k = 0; k < 3; ++k) sc[k] += diffuse * L.diff[k] * cc[k];
     Vec3 hv = 0.5f * (view + ld);
-    {
-      const float m = sqrtf (dot (hv, hv));
-      hv = make3 (hv.x / m, hv.y / m, hv.z / m);
-    }
+    hv = (1.f / sqrtf (dot (hv, hv))) * hv;
     if (dot (g, hv) < 0.f) g = make3 (-g.x, -g.y, -g.z);
     const float doth = clampf (dot (g, hv), 0.f, 1.f);
     const float intensity = powf (doth, L.spec_pow);
