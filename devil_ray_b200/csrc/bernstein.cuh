@@ -336,26 +336,32 @@ struct LU3
     }
   }
 
-  // x with the transposed matrix: U^T z = b, L^T w = z, x = P^T w.
-  DRB_D void solve_transposed (const float (&b)[3], float (&x)[3]) const
+  // x = g A^-1 by the columns of the inverse (matrix_inverse, matrix.hpp:430-456),
+  // the same sums and quotients as solve () of the three unit vectors followed
+  // by the products with g; what a unit vector's zeros make zero is left out,
+  // three of the nine divisions among it.
+  DRB_D void times_inverse (const float (&g)[3], float (&x)[3]) const
   {
-    float w[3];
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+    for (int k = 0; k < 3; ++k)
     {
-      w[r] = b[r];
+      // the column of the inverse for row k of the permuted matrix
+      float y[3] = { 0.f, 0.f, 0.f };
+      y[k] = 1.f / a[k][k];
 #pragma unroll
-      for (int c = 0; c < r; ++c) w[r] -= a[c][r] * w[c];
+      for (int r = k + 1; r < 3; ++r)
+      {
+#pragma unroll
+        for (int c = k; c < r; ++c) y[r] -= a[r][c] * y[c];
+        y[r] = y[r] / a[r][r];
+      }
+      float col[3];
+      back_substitute (y, col);
+      const float s = g[0] * col[0] + g[1] * col[1] + g[2] * col[2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (perm[k] == i) x[i] = s;
     }
-#pragma unroll
-    for (int r = 2; r >= 0; --r)
-    {
-#pragma unroll
-      for (int c = r + 1; c < 3; ++c) w[r] -= a[c][r] * w[c];
-      w[r] = w[r] / a[r][r];
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) x[i] = perm[0] == i ? w[0] : (perm[1] == i ? w[1] : w[2]);
   }
 };
 

@@ -406,19 +406,24 @@ DRB_D float4 shade_sample (const VolumeParams &vp, int el, const float (&r)[3], 
   if (!vp.use_lighting) return c;
   float4 acc = make_float4 (0.f, 0.f, 0.f, 0.f);
   if (!(c.w > 0.01f)) return acc;
-  // gradient = gref * J^-1 (the reference multiplies by the inverse,
-  // matrix.hpp:430-456): one solve with the transposed factors
+  // gradient = gref * J^-1
   float gw[3];
-  lu.solve_transposed (gref, gw);
+  lu.times_inverse (gref, gw);
   Vec3 g = make3 (gw[0], gw[1], gw[2]);
-  g = (1.f / sqrtf (dot (g, g))) * g;
+  {
+    const float m = sqrtf (dot (g, g));
+    g = make3 (g.x / m, g.y / m, g.z / m);
+  }
   const Vec3 view = make3 (-ray.dir.x, -ray.dir.y, -ray.dir.z);
   const Vec3 wp = make3 (wpos[0], wpos[1], wpos[2]);
   for (int l = 0; l < vp.n_lights; ++l)
   {
     const PointLight L = vp.lights[l];
     Vec3 ld = make3 (L.pos[0] - wp.x, L.pos[1] - wp.y, L.pos[2] - wp.z);
-    ld = (1.f / sqrtf (dot (ld, ld))) * ld;
+    {
+      const float m = sqrtf (dot (ld, ld));
+      ld = make3 (ld.x / m, ld.y / m, ld.z / m);
+    }
     if (dot (ld, g) < 0.f) g = make3 (-g.x, -g.y, -g.z);
     const float diffuse = clampf (dot (ld, g), 0.f, 1.f);
     float sc[4] = { L.amb[0] * c.x, L.amb[1] * c.y, L.amb[2] * c.z, c.w };
@@ -426,7 +431,10 @@ DRB_D float4 shade_sample (const VolumeParams &vp, int el, const float (&r)[3], 
 #pragma unroll
     for (int k = 0; k < 3; ++k) sc[k] += diffuse * L.diff[k] * cc[k];
     Vec3 hv = 0.5f * (view + ld);
-    hv = (1.f / sqrtf (dot (hv, hv))) * hv;
+    {
+      const float m = sqrtf (dot (hv, hv));
+      hv = make3 (hv.x / m, hv.y / m, hv.z / m);
+    }
     if (dot (g, hv) < 0.f) g = make3 (-g.x, -g.y, -g.z);
     const float doth = clampf (dot (g, hv), 0.f, 1.f);
     const float intensity = powf (doth, L.spec_pow);
