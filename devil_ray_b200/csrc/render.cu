@@ -23,6 +23,7 @@
 #include "drb_internal.h"
 #include "locate.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -782,12 +783,16 @@ DRB_D void keep_sample (const VolumeParams &vp, RayMarch &s, int el, const float
 // locate (coherent or full), shade, take_sample.
 // Partials go to slot 5 i + segment of ray i and the framebuffer pixel gets
 // their front-to-back composite, so the processing order changes nothing.
-template <int P, bool WIDE, int S>
+// FEW: the first part of the plain march of few rays (volume_group_kernel): a
+// ray is put aside, as it stands, in left[its index] after its first sample whose
+// alpha is below `opaque`; rays that end here leave an index of -1 there.
+template <int P, bool WIDE, int S, bool FEW>
 __global__ void __launch_bounds__ (128)
 volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *__restrict__ queue,
                VolumePartial *__restrict__ partials, float4 *__restrict__ fb_color,
                float *__restrict__ fb_depth, int *__restrict__ ray_samples,
-               int *__restrict__ ray_iters, int *__restrict__ ray_cands)
+               int *__restrict__ ray_iters, int *__restrict__ ray_cands, RayMarch *__restrict__ left,
+               float opaque)
 {
   constexpr int kChunk = 32;
   const unsigned FULL = 0xffffffffu;
@@ -828,7 +833,11 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
         step[0] = s.ray.dir.x * vp.sample_dist;
         step[1] = s.ray.dir.y * vp.sample_dist;
         step[2] = s.ray.dir.z * vp.sample_dist;
-        if (!live) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+        if (!live)
+        {
+          if (FEW) left[s.i].i = -1;
+          finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+        }
       }
       pool_next += min (__popc (need), avail);
       need = __ballot_sync (FULL, s.i < 0);
@@ -846,8 +855,16 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
     float4 sc = make_float4 (0.f, 0.f, 0.f, 0.f);
     if (el >= 0) sc = shade_sample<P, S> (vp, el, ref, s.ray, lu, pt);
     keep_sample (vp, s, el, ref);
+    const int i = s.i;
     if (take_sample (s, el >= 0, sc, vp.sample_dist, partials))
       finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
+    else if (FEW && !(el >= 0 && sc.w >= opaque))
+    {
+      left[i] = s;
+      s.i = -1;
+      continue;
+    }
+    if (FEW && s.i < 0) left[i].i = -1;
   }
 }
 
@@ -857,13 +874,16 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
 // each lane repeating the same steps on values passed by shuffle, so the
 // result is the one-lane march's bit for bit (a plain sample does not depend
 // on the one before it, and the distances are the same repeated sums).
-// Samples behind the one that ends the ray are thrown away.  Bound, like the
+// Samples behind the one that ends the ray are thrown away.  A group's round
+// takes several times a lane's sample, so a ray that ends within a few samples
+// loses by it: the rays come, in left, from volume_kernel's first part, which
+// keeps the rays whose samples are so opaque that they end soon.  Bound, like the
 // one-lane march, by the chains of node loads and Newton steps; the lanes give
-// the SMs enough of them.  256^2 pixels, 500 samples, 8^3 order-2 hexes: 4.32
-// -> 2.06 ms a frame.
+// the SMs enough of them.  256^2 pixels, 500 samples, 8^3 order-2 hexes: 4.38 ->
+// 1.99 ms a frame.
 template <int P, bool WIDE, int S>
 __global__ void __launch_bounds__ (128)
-volume_group_kernel (VolumeParams vp, int G, const Ray *__restrict__ rays, int n_rays,
+volume_group_kernel (VolumeParams vp, int G, const RayMarch *__restrict__ left, int n_rays,
                      int *__restrict__ queue, VolumePartial *__restrict__ partials,
                      float4 *__restrict__ fb_color, float *__restrict__ fb_depth,
                      int *__restrict__ ray_samples, int *__restrict__ ray_iters,
@@ -889,13 +909,8 @@ volume_group_kernel (VolumeParams vp, int G, const Ray *__restrict__ rays, int n
       const int i = base + __popc (need & ((1u << lead) - 1u));
       if (s.i < 0 && i < n_rays)
       {
-        s.i = i;
-        s.ray = rays[i];
-        if (!start_ray (vp, s))
-        {
-          if (g == 0) finish_ray (s, fb_color, fb_depth, ray_samples, ray_iters, ray_cands);
-          s.i = -1;
-        }
+        s = left[i];                       // .i is -1 where the ray has ended
+        if (g != 0) s.iters = s.cands = 0; // counted once a group
       }
       need = __ballot_sync (FULL, s.i < 0 && g == 0);
     }
@@ -1088,29 +1103,49 @@ int group_lanes (const VolumeParams &vp, int n)
   return G;
 }
 
+// Blocks of 128 threads for a march by `lanes` lanes: the resident ones.
+template <class K> unsigned march_blocks (K kernel, long long lanes)
+{
+  int nb = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, kernel, 128, 0);
+  const long long blocks = (long long)std::max (nb, 1) * sm_count ();
+  return (unsigned)std::max (1ll, std::min (blocks, (lanes + 127) / 128));
+}
+
+// queue: kVolumeQueue ints, zero (the queues of the two parts of a march).
+constexpr int kVolumeQueue = 2;
+
+// Alpha of a sample from which a ray stays with one lane: rays of such samples
+// reach 0.95 within about 192 / G of them, less than a group's first round
+// costs.  Measured (us a frame, 256^2 pixels, 8 lanes, all rays with one lane /
+// all with groups / by this rule), 8^3 order-2 hexes, sample alpha 0.05: 850 /
+// 465 / 481, 0.25: 334 / 356 / 280, 1: 102 / 240 / 107; 8^3 x 6 order-2 tets,
+// 0.05: 3858 / 2624 / 2746, 0.25: 1192 / 1617 / 1086, 1: 181 / 1069 / 195.
+// 128^2, 32 lanes, the hexes, 0.3: 243 / 220 / 243, 1: 104 / 222 / 113.
+float group_opaque (int G) { return G / 64.f; }
+
 template <int P, bool WIDE, int S>
 int launch_volume_w (const VolumeParams &vp, const Ray *rays, int n, int *queue,
                      VolumePartial *partials, float4 *fb, float *depth, const drb_ray_stats &st,
                      cudaStream_t s)
 {
-  int nb = 0;
   const int G = group_lanes (vp, n);
-  if (G > 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, volume_group_kernel<P, WIDE, S>, 128, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor (&nb, volume_kernel<P, WIDE, S>, 128, 0);
-  if (nb < 1) nb = 1;
-  long long blocks = (long long)nb * sm_count ();
-  const long long need = ((long long)n * G + 127) / 128;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) blocks = 1;
-  if (G > 1)
+  if (G == 1)
   {
-    volume_group_kernel<P, WIDE, S><<<(unsigned)blocks, 128, 0, s>>> (
-        vp, G, rays, n, queue, partials, fb, depth, st.samples, st.iters, st.candidates);
-    return check_launch ("volume_group_kernel");
+    volume_kernel<P, WIDE, S, false><<<march_blocks (volume_kernel<P, WIDE, S, false>, n), 128, 0, s>>> (
+        vp, rays, n, queue, partials, fb, depth, st.samples, st.iters, st.candidates, nullptr, 0.f);
+    return check_launch ("volume_kernel");
   }
-  volume_kernel<P, WIDE, S><<<(unsigned)blocks, 128, 0, s>>> (vp, rays, n, queue, partials, fb, depth,
-                                                              st.samples, st.iters, st.candidates);
-  return check_launch ("volume_kernel");
+  Scratch scr (s);
+  RayMarch *left = scr.alloc<RayMarch> (n);
+  if (!left) return status_from (scr.err);
+  volume_kernel<P, WIDE, S, true><<<march_blocks (volume_kernel<P, WIDE, S, true>, n), 128, 0, s>>> (
+      vp, rays, n, queue, partials, fb, depth, st.samples, st.iters, st.candidates, left, group_opaque (G));
+  if (int e = check_launch ("volume_kernel")) return e;
+  volume_group_kernel<P, WIDE, S>
+      <<<march_blocks (volume_group_kernel<P, WIDE, S>, (long long)n * G), 128, 0, s>>> (
+          vp, G, left, n, queue + 1, partials, fb, depth, st.samples, st.iters, st.candidates);
+  return check_launch ("volume_group_kernel");
 }
 
 // full locates of the march walk the 4-wide tree when the BVH has one
@@ -1432,11 +1467,11 @@ extern "C" int drb_volume_integrate (const drb_mesh *mesh, const drb_mesh *field
   int *flags = scr.alloc<int> (np);
   int *offs = scr.alloc<int> (np);
   int *total = scr.alloc<int> (1);
-  int *queue = scr.alloc<int> (1);
+  int *queue = scr.alloc<int> (kVolumeQueue);
   if (scr.err != cudaSuccess) return status_from (scr.err);
   init_partials_kernel<<<div_up (np, 256), 256, 0, s>>> (raw, np);
   if ((st = check_launch ("init_partials_kernel"))) return st;
-  cudaMemsetAsync (queue, 0, sizeof (int), s);
+  cudaMemsetAsync (queue, 0, kVolumeQueue * sizeof (int), s);
   const Ray *rays = (const Ray *)active_rays;
   st = launch_volume (mesh, vp, rays, n_rays, queue, raw, nullptr, nullptr, stats, s);
   if (st) return st;
@@ -1473,9 +1508,9 @@ extern "C" int drb_volume_render (const drb_mesh *mesh, const drb_mesh *field, c
   if (n_rays == 0) return DRB_OK;
   cudaStream_t s = (cudaStream_t)stream;
   Scratch scr (s);
-  int *queue = scr.alloc<int> (1);
+  int *queue = scr.alloc<int> (kVolumeQueue);
   if (!queue) return status_from (scr.err);
-  cudaMemsetAsync (queue, 0, sizeof (int), s);
+  cudaMemsetAsync (queue, 0, kVolumeQueue * sizeof (int), s);
   const Ray *rays = (const Ray *)active_rays;
   float4 *fb = (float4 *)fb_rgba;
   st = launch_volume (mesh, vp, rays, n_rays, queue, nullptr, fb, fb_depth, stats, s);

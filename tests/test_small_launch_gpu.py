@@ -46,7 +46,9 @@ def test_few_rays_equal_many(cuda, kind, p, lit):
     light = [render.PointLight.default(camera)]
     active = render.cull_rays(camera.create_rays(cuda), mesh.bounds())
     assert active.shape[0] > 37888
-    for opacity in (0.02, 0.9):
+    # at the larger opacities rays end within a few samples, some of them
+    # before their group would take them over
+    for opacity in (0.02, 0.9, 0.9999, 1.0):
         vol = render.Volume(mesh, field)
         table = render.ColorTable()
         table.add_point(0.0, (0.1, 0.2, 0.9))
