@@ -737,9 +737,12 @@ LaunchShape persistent_shape (const drb_mesh *mesh, const drb_bvh *bvh, const dr
   return { (int)blocks, cfg.block, cfg.chunk };
 }
 
-// Small batches: up to kSmallPerSm queries an SM take one launch of 64-thread
-// blocks without query order or queue; each warp takes one chunk of 1 to 32
-// queries, kSmallWarps warps an SM before the chunks grow.  Such a batch is
+// Small batches: without a configuration or an order of the caller's, up to
+// kSmallPerSm queries an SM take one launch of 64-thread blocks without query
+// order or queue; each warp takes one chunk of 1 to 32 queries, kSmallWarps
+// warps an SM before the chunks grow.  (A configuration is a promise about the
+// launch: blocks per SM to leave room for other work, the row mode, the query
+// order.  It holds at every size.)  Such a batch is
 // bound by its slowest query's chain of node loads and Newton steps and by
 // launches: 64 queries a warp ran the sum of two rounds of the slowest lanes,
 // and the order cost five launches.  Measured (us a call, ordered / this):
@@ -752,7 +755,10 @@ constexpr int kSmallPerSm = 700;
 constexpr int kSmallWarps = 16;
 constexpr int kSmallBlock = 64;
 
-bool small_batch (int n) { return n <= kSmallPerSm * sm_count (); }
+bool small_batch (const drb_locate_config *cfg, int n)
+{
+  return !cfg && n <= kSmallPerSm * sm_count ();
+}
 
 LaunchShape small_batch_shape (int n)
 {
@@ -819,7 +825,7 @@ int locate_batched_impl (const drb_mesh *mesh, const drb_bvh *bvh, const float *
   if (n == 0) return DRB_OK;
   const drb_locate_config cfg = cfg_in ? *cfg_in : default_config (mesh->order);
   if ((st = check_config (cfg))) return st;
-  if (!order_in && small_batch (n))
+  if (!order_in && small_batch (cfg_in, n))
     return launch_small (mesh, bvh, pts, n, opts, cell, ref, stats, s);
   Scratch scr (s);
   int *head = scr.alloc<int> (1);
@@ -861,7 +867,7 @@ int locate_batched_impl (const drb_mesh *mesh, const drb_bvh *bvh, const float *
 }
 
 // Same as locate_batched_impl with sorting (queries read through the index
-// order), but over caller-provided workspace.
+// order), but over caller-provided workspace.  cfg_in NULL: the default.
 int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pts, int n,
                        const drb_newton_opts *opts, const drb_locate_config *cfg_in,
                        const LocateWorkspace &ws, int *cell, float *ref, drb_query_stats stats,
@@ -872,7 +878,7 @@ int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pt
   if (n == 0) return DRB_OK;
   const drb_locate_config cfg = cfg_in ? *cfg_in : default_config (mesh->order);
   if ((st = check_config (cfg))) return st;
-  if (small_batch (n)) return launch_small (mesh, bvh, pts, n, opts, cell, ref, stats, s);
+  if (small_batch (cfg_in, n)) return launch_small (mesh, bvh, pts, n, opts, cell, ref, stats, s);
   const int *ord = nullptr;
   if (cfg.sort_queries)
   {

@@ -130,8 +130,12 @@ extern "C" int drb_locate_host (const drb_mesh *mesh, const drb_bvh *bvh, const 
   {
     st = status_from (e);
   }
-  drb_locate_config c = cfg ? *cfg : drb_locate_config{ 128, 0, 64, 1, 0 };
-  c.sort_queries = 1; // the workspace path sorts each chunk
+  drb_locate_config c;
+  if (cfg)
+  {
+    c = *cfg;
+    c.sort_queries = 1; // the workspace path sorts each chunk
+  }
   for (long long off = 0, k = 0; off < n && st == DRB_OK; off += chunk, ++k)
   {
     Lane &L = lane[k % kLanes];
@@ -140,7 +144,7 @@ extern "C" int drb_locate_host (const drb_mesh *mesh, const drb_bvh *bvh, const 
                          cudaMemcpyHostToDevice, L.s);
     if (e == cudaSuccess)
     {
-      st = locate_batched_ws (mesh, bvh, L.pts, m, opts, &c, L.ws, L.cell, L.ref,
+      st = locate_batched_ws (mesh, bvh, L.pts, m, opts, cfg ? &c : nullptr, L.ws, L.cell, L.ref,
                               drb_query_stats{ nullptr, nullptr, nullptr }, L.s);
       if (st) break;
       e = cudaMemcpyAsync (host_cell + off, L.cell, sizeof (int) * (size_t)m,

@@ -328,7 +328,10 @@ typedef struct drb_locate_config
 /* Batched point location, same results as drb_locate (same traversal order
  * and per-candidate solves per point): queries Morton-sorted, persistent
  * warps popping chunks from a global atomic queue, idle lanes refilled by
- * ballot ranking, Newton solves of a warp run converged.  cfg NULL = default.
+ * ballot ranking, Newton solves of a warp run converged.  cfg NULL = the
+ * library's choice: the default configuration { 128, 0, 64, 1, 0 }, or for a
+ * small batch (up to 700 queries per SM) one launch without order or queue.  A
+ * configuration that is given holds at every size.
  * Replaces UnstructuredMesh::locate (data_model/unstructured_mesh.cpp:124-148). */
 int drb_locate_batched (const drb_mesh *mesh, const drb_bvh *bvh, const float *pts, int n,
                         const drb_newton_opts *opts, const drb_locate_config *cfg, int *cell,

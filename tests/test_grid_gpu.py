@@ -74,9 +74,17 @@ def test_grid_lists_match_restatement(cuda, name, scale):
     print(f"{name}: {dims} cells, {keys.size} entries, {keys.size / n_cells:.2f} per cell")
 
 
+def _launch(name):
+    """Configuration of a batch that few queries would take one launch for
+    (small); a given one keeps the persistent kernel and its query order."""
+    from devil_ray_b200 import _lib as L
+    return None if name == "small" else L.DrbLocateConfig(128, 0, 64, 1, 0)
+
+
 @pytest.mark.parametrize("name", ["trilinear_12", "p3_10", "p1_9", "tet_p2"])
 @pytest.mark.parametrize("scale", [0.5, 1.0, 3.0])
-def test_grid_locate_equals_tree(cuda, name, scale):
+@pytest.mark.parametrize("launch", ["small", "persistent"])
+def test_grid_locate_equals_tree(cuda, name, scale, launch):
     import torch
     from devil_ray_b200 import _lib as L
     from devil_ray_b200 import api, meshgen
@@ -91,7 +99,8 @@ def test_grid_locate_equals_tree(cuda, name, scale):
         for b in (tree, grid):
             if mode == L.GUESS_SUBBOX_LINEAR and b.leaf_maps is None:
                 b.build_leaf_maps(g)
-            loc = api.BatchedLocator(g, tol=1e-5, max_steps=20, guess_mode=mode, bvh=b)
+            loc = api.BatchedLocator(g, tol=1e-5, max_steps=20, guess_mode=mode, bvh=b,
+                                     config=_launch(launch))
             out.append(loc.locate(q, stats=True))
         torch.cuda.synchronize()
         (c0, r0, i0, a0, _), (c1, r1, i1, a1, n1) = out
@@ -140,7 +149,8 @@ def test_grid_locate_edge_cases(cuda):
 
 
 @pytest.mark.parametrize("kind", ["quad", "tri"])
-def test_grid_locate_equals_tree_2d(cuda, kind):
+@pytest.mark.parametrize("launch", ["small", "persistent"])
+def test_grid_locate_equals_tree_2d(cuda, kind, launch):
     """2D quad and triangle meshes (their boxes are flat in z, so the grid
     has one cell across z): grid and tree give the same answers bit for
     bit, with queries on and off the mesh plane."""
@@ -158,8 +168,10 @@ def test_grid_locate_equals_tree_2d(cuda, kind):
     z = np.where(rng.random(50000) < 0.9, 0.0, 0.01)
     q = np.concatenate([xy, z[:, None]], 1).astype(np.float32)
     bvh = g.get_bvh()
-    tree = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=bvh.without_grid())
-    grid = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=bvh.without_grid().build_grid(1.0))
+    tree = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=bvh.without_grid(),
+                              config=_launch(launch))
+    grid = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=bvh.without_grid().build_grid(1.0),
+                              config=_launch(launch))
     c0, r0, i0, a0, _ = tree.locate(q, stats=True)
     c1, r1, i1, a1, _ = grid.locate(q, stats=True)
     torch.cuda.synchronize()

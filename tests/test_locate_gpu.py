@@ -158,18 +158,27 @@ def test_local_frame_locates_fine_order3_mesh(cuda):
           f"absolute-coordinate FP32 Newton misses {(ac < 0).sum()} of {len(q)}")
 
 
+def _launch(name):
+    """Configuration of a batch that few queries would take one launch for
+    (small); a given one keeps the persistent kernel and its query order."""
+    from devil_ray_b200 import _lib as L
+    return None if name == "small" else L.DrbLocateConfig(128, 0, 64, 1, 0)
+
+
 @pytest.mark.parametrize("name", ["volume_8", "p3_10", "p1_9"])
-def test_wide_traversal_equals_binary(cuda, name):
-    """The batched kernel over the 4-wide tree returns exactly what it
-    returns over the binary tree: cells, reference points (bit for bit),
+@pytest.mark.parametrize("launch", ["small", "persistent"])
+def test_wide_traversal_equals_binary(cuda, name, launch):
+    """The batched kernels over the 4-wide tree return exactly what they
+    return over the binary tree: cells, reference points (bit for bit),
     Newton iterations and candidate counts; only node visits differ."""
     import torch
     from devil_ray_b200 import api
     m, q, g = _setup(cuda, name, 50000, 13)
     b = g.get_bvh()
     assert b.wide_nodes is not None
-    wide = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=b)
-    binary = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=b.binary_only())
+    wide = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=b, config=_launch(launch))
+    binary = api.BatchedLocator(g, tol=1e-5, max_steps=20, bvh=b.binary_only(),
+                                config=_launch(launch))
     c0, r0, i0, a0, n0 = binary.locate(q, stats=True)
     c1, r1, i1, a1, n1 = wide.locate(q, stats=True)
     torch.cuda.synchronize()
@@ -180,14 +189,15 @@ def test_wide_traversal_equals_binary(cuda, name):
           f"wide {n1.float().mean().item():.2f}")
 
 
-def test_locate_host_equals_device_batched(cuda):
+@pytest.mark.parametrize("launch", ["small", "persistent"])
+def test_locate_host_equals_device_batched(cuda, launch):
     """drb_locate_host (chunked, copies overlapped on three streams) gives
     the batched locate's results, for chunk sizes that do and do not divide
     the batch."""
     import torch
     from devil_ray_b200 import api
     m, q, g = _setup(cuda, "volume_8", 100000, 17)
-    loc = api.BatchedLocator(g, tol=1e-5, max_steps=20)
+    loc = api.BatchedLocator(g, tol=1e-5, max_steps=20, config=_launch(launch))
     c0, r0 = loc.locate(q)
     torch.cuda.synchronize()
     hq = torch.from_numpy(np.ascontiguousarray(q, np.float32)).pin_memory()
@@ -224,7 +234,8 @@ def test_row_modes_identical(cuda, name):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", ["hex", "tet"])
-def test_locate_graph_replay_matches_eager(cuda, shape):
+@pytest.mark.parametrize("launch", ["small", "persistent"])
+def test_locate_graph_replay_matches_eager(cuda, shape, launch):
     """The batched locate captured into a CUDA graph (BatchedLocator.capture)
     gives the eager results bit for bit on new queries at every replay."""
     import torch
@@ -236,7 +247,7 @@ def test_locate_graph_replay_matches_eager(cuda, shape):
     else:
         m = meshgen.tet_warped_mesh(6, 2, 0.05, jitter=0.01, seed=5)
         g = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda, shape=L.SHAPE_SIMPLEX)
-    loc = api.BatchedLocator(g, tol=1e-5, max_steps=20)
+    loc = api.BatchedLocator(g, tol=1e-5, max_steps=20, config=_launch(launch))
     n = 50000
     lg = loc.capture(n)
     for seed in (3, 4, 5):
@@ -253,9 +264,9 @@ def test_locate_graph_replay_matches_eager(cuda, shape):
 @pytest.mark.parametrize("name", ["volume_8", "p3_10", "p1_9"])
 @pytest.mark.parametrize("guess", ["centre", "subref"])
 def test_staged_equals_ordered_and_plain(cuda, name, guess):
-    """Every placement of the queries and results (read through the Morton
-    order, staged records, staged results) and the caller-ordered path
-    (drb_locate_ordered) give the plain one-thread-per-query kernel's
+    """The small batch's launch, every placement of the queries and results
+    (read through the Morton order, staged records, staged results) and the
+    caller-ordered path (drb_locate_ordered) give the plain one-thread-per-query kernel's
     answers bit for bit, statistics included."""
     import torch
     from devil_ray_b200 import _lib as L
@@ -267,10 +278,10 @@ def test_staged_equals_ordered_and_plain(cuda, name, guess):
     order = loc.order(q)
     c1, r1, i1, a1, n1 = loc.locate(q, order=order, stats=True)
     c2, r2 = g.locate(q, tol=1e-5, max_steps=20, guess_mode=mode)
-    # query records staged first (sort_queries 2), results staged as well
-    # and put back by a separate pass (3)
+    # read through the order (sort_queries 1), query records staged first (2),
+    # results staged as well and put back by a separate pass (3)
     out = []
-    for mode_s in (2, 3):
+    for mode_s in (1, 2, 3):
         loc_s = api.BatchedLocator(g, tol=1e-5, max_steps=20, guess_mode=mode,
                                    config=L.DrbLocateConfig(128, 0, 64, mode_s, 0))
         out.append(loc_s.locate(q, stats=True))

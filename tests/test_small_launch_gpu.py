@@ -78,3 +78,42 @@ def test_few_rays_equal_many(cuda, kind, p, lit):
         done = torch.isfinite(seen)
         assert done.sum() > 1000
         assert torch.equal(parts[done], colors[done]) and torch.equal(seen[done], depths[done])
+
+
+# a configuration that is given decides the launch at every size: with the
+# order there are launches before the locate kernel, with staged results one
+# behind it, without order or configuration there is one in all
+@pytest.mark.parametrize("entry", ["batched", "noalloc"])
+def test_a_given_configuration_holds_for_few_queries(cuda, entry):
+    import ctypes as C
+    import torch
+    m, shape = _mesh("hex", 5, 2)
+    g = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda, shape=shape)
+    q = torch.as_tensor(meshgen.uniform_queries(5000, 3), device=cuda)
+    bd = g.get_bvh().desc()
+    md = g.desc()
+    opts = L.DrbNewtonOpts(1e-5, 20, L.GUESS_ELEM_CENTER, None)
+    fn = L.lib().drb_locate_batched if entry == "batched" else L.lib().drb_locate_batched_noalloc
+    out = []
+
+    def launches(cfg):
+        cell = torch.empty(5000, dtype=torch.int32, device=cuda)
+        ref = torch.empty((5000, 3), dtype=torch.float32, device=cuda)
+        first = L.lib().drb_kernel_launches()
+        assert fn(C.byref(md), C.byref(bd), C.c_void_p(q.data_ptr()), 5000, C.byref(opts),
+                  None if cfg is None else C.byref(cfg), C.c_void_p(cell.data_ptr()),
+                  C.c_void_p(ref.data_ptr()), L.DrbQueryStats(),
+                  C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        out.append((cell, ref))
+        return L.lib().drb_kernel_launches() - first
+
+    assert launches(None) == 1
+    ordered = launches(L.DrbLocateConfig(128, 0, 64, 1, 0))
+    assert ordered > 1
+    if entry == "batched":
+        staged = launches(L.DrbLocateConfig(128, 0, 64, 2, 0))
+        assert launches(L.DrbLocateConfig(128, 0, 64, 3, 0)) == staged + 1
+    assert launches(L.DrbLocateConfig(128, 1, 64, 0, 1)) == 1
+    for cell, ref in out[1:]:
+        assert torch.equal(cell, out[0][0])
+        assert torch.equal(ref.view(torch.int32), out[0][1].view(torch.int32))

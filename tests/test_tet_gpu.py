@@ -596,12 +596,15 @@ def test_tet_surface_curved_faces_lie_on_rays(cuda, p):
 
 @pytest.mark.parametrize("p", ORDERS)
 @pytest.mark.parametrize("guess", ["zero", "center", "subref"])
-def test_tet_batched_skips_only_failing_solves(cuda, p, guess):
+@pytest.mark.parametrize("given", [False, True])
+def test_tet_batched_skips_only_failing_solves(cuda, p, guess, given):
     """The batched locate skips a candidate tet whose solve already failed
     for the query (leaf-independent guesses) and tets whose hull planes
     reject the query. Against the plain kernel, which solves every
     candidate: the same cells and reference points bit for bit, the same
-    candidate counts, and never more Newton steps for any query."""
+    candidate counts, and never more Newton steps for any query.  A given
+    configuration keeps the persistent kernel; without one so few queries
+    take one launch."""
     import torch
     from devil_ray_b200 import _lib as L
     from devil_ray_b200 import api, meshgen
@@ -611,7 +614,8 @@ def test_tet_batched_skips_only_failing_solves(cuda, p, guess):
             "subref": L.GUESS_SUBREF_CENTER}[guess]
     pts = torch.as_tensor(meshgen.uniform_queries(60000, 91 + p), device=cuda)
     c0, r0, it0, ca0, _ = g.locate(pts, tol=1e-5, max_steps=20, guess_mode=mode, stats=True)
-    bl = api.BatchedLocator(g, tol=1e-5, max_steps=20, guess_mode=mode)
+    config = L.DrbLocateConfig(128, 0, 64, 1, 0) if given else None
+    bl = api.BatchedLocator(g, tol=1e-5, max_steps=20, guess_mode=mode, config=config)
     c1, r1, it1, ca1, _ = bl.locate(pts, stats=True)
     torch.cuda.synchronize()
     assert torch.equal(c0, c1)
