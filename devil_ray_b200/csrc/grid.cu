@@ -213,7 +213,8 @@ __global__ void cell_fill_kernel (GridGeom g, const float4 *__restrict__ table, 
 
 // The lists in leaf order: a warp takes 32 consecutive cells, a lane an
 // entry, whose place is the number of smaller ones in its cell's list (a
-// leaf occurs once in a list).  The list is re-read through L1.
+// leaf occurs once in a list).  The list is re-read through L1.  Entry indices
+// are unsigned: the last round's reach past the end, which is below 2^31.
 __global__ void cell_order_kernel (const int *__restrict__ start, long long n_cells,
                                    const int *__restrict__ lists, int *__restrict__ entries)
 {
@@ -221,24 +222,24 @@ __global__ void cell_order_kernel (const int *__restrict__ start, long long n_ce
   const int lane = threadIdx.x & 31;
   const long long c0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) - lane;
   if (c0 >= n_cells) return;
-  const int lo = __ldg (start + min (c0 + lane, n_cells));
-  const int end = __ldg (start + min (c0 + 32, n_cells));
-  const int begin = __shfl_sync (FULL, lo, 0);
-  for (int base = begin; base < end; base += 32)
+  const unsigned lo = __ldg (start + min (c0 + lane, n_cells));
+  const unsigned end = __ldg (start + min (c0 + 32, n_cells));
+  const unsigned begin = __shfl_sync (FULL, lo, 0);
+  for (unsigned base = begin; base < end; base += 32)
   {
-    const int e = base + lane;
+    const unsigned e = base + lane;
     int j = 0; // the last cell that starts at or before e
 #pragma unroll
     for (int h = 16; h; h >>= 1)
       if (__shfl_sync (FULL, lo, j + h) <= e) j += h;
-    const int first = __shfl_sync (FULL, lo, j);
-    const int next = __shfl_sync (FULL, lo, (j + 1) & 31);
-    const int last = j == 31 ? end : next;
+    const unsigned first = __shfl_sync (FULL, lo, j);
+    const unsigned next = __shfl_sync (FULL, lo, (j + 1) & 31);
+    const unsigned last = j == 31 ? end : next;
     if (e < end)
     {
       const int v = __ldg (lists + e);
       int rank = 0;
-      for (int q = first; q < last; ++q) rank += __ldg (lists + q) < v;
+      for (unsigned q = first; q < last; ++q) rank += __ldg (lists + q) < v;
       entries[first + rank] = v;
     }
   }

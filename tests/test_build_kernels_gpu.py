@@ -302,3 +302,49 @@ def test_grid_lists_of_every_length(cuda, n, scale):
     start = np.searchsorted(cell[order], np.arange(n_cells + 1))
     assert np.array_equal(b.grid_start.cpu().numpy(), start)
     assert np.array_equal(b.grid_entries.cpu().numpy(), leaf[order])
+
+
+def test_grid_lists_just_below_the_entry_limit(cuda):
+    """2^31 - 2 entries, the largest count below the limit that rows of
+    equal lists make: 9,513 rows of 3,641 cells, 62 leaves a row.  Entry
+    indices run past what a signed index plus one warp holds.  (17 GB.)"""
+    import torch
+    from devil_ray_b200 import _lib as L
+    dims, per_row = (3641, 151, 63), 62
+    rows = dims[1] * dims[2]
+    n_cells, n = rows * dims[0], rows * per_row
+    m = n_cells * per_row
+    assert m == 2**31 - 2
+    if torch.cuda.mem_get_info(cuda)[0] < 24 << 30:
+        pytest.skip("needs 24 GB of device memory")
+    # node records that hold two leaves each (the others hold none)
+    row = torch.arange(n, device=cuda) // per_row
+    y, z = (row % dims[1]).float(), (row // dims[1]).float()
+    lo = torch.stack([torch.full_like(y, 0.5), y + 0.25, z + 0.25], 1)
+    hi = torch.stack([torch.full_like(y, dims[0] - 0.5), y + 0.75, z + 0.75], 1)
+    rec = torch.zeros((n - 1, 16), dtype=torch.float32, device=cuda)
+    rec[:n // 2, :12] = torch.cat([lo, hi], 1).reshape(n // 2, 12)
+    rec.view(torch.int32)[:n // 2, 12:14] = -1 - torch.arange(n, dtype=torch.int32,
+                                                             device=cuda).reshape(-1, 2)
+    leaf_nodes = torch.arange(n, dtype=torch.int32, device=cuda)
+    start = torch.empty(n_cells + 1, dtype=torch.int32, device=cuda)
+    entries = torch.full((m,), -1, dtype=torch.int32, device=cuda)
+    boxes = torch.empty((n, 8), dtype=torch.float32, device=cuda)
+    d = L.DrbBvh()
+    d.n_inner, d.n_leaf = n - 1, n
+    d.inner_nodes, d.leaf_nodes = rec.data_ptr(), leaf_nodes.data_ptr()
+    d.grid_start, d.grid_entries, d.grid_boxes = (t.data_ptr() for t in (start, entries, boxes))
+    for q in range(3):
+        d.grid_dims[q], d.grid_origin[q], d.grid_inv[q] = dims[q], 0.0, 1.0
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    L.check(L.lib().drb_bvh_grid_build(C.byref(d), s), "drb_bvh_grid_build")
+    want = per_row * torch.arange(n_cells + 1, dtype=torch.int64, device=cuda)
+    assert torch.equal(start.long(), want)
+    del want
+    lists = entries.reshape(rows, dims[0], per_row)
+    leaves = torch.arange(n, dtype=torch.int32, device=cuda).reshape(rows, 1, per_row)
+    for r in range(0, rows, 500):
+        assert torch.equal(lists[r:r + 500],
+                           leaves[r:r + 500].expand(-1, dims[0], -1)), f"row {r}"
+    del entries, lists
+    torch.cuda.empty_cache()
