@@ -272,13 +272,18 @@ def test_wide_plan_and_emit(cuda, kind, n_elem):
 
 
 # scales: lists of a few leaves, of some tens, of about a hundred (more than
-# 64 comparisons an entry: radix passes), and one cell with every leaf
-@pytest.mark.parametrize("n,scale", [(3, 0.4), (5, 1.0), (9, 2.6), (9, 5.0), (4, 1e6)])
-def test_grid_lists_of_every_length(cuda, n, scale):
+# 64 comparisons an entry: radix passes), and one cell with every leaf (more
+# than 64 leaves a cell: radix passes at once).  power: control points raised
+# to it, so that leaves crowd into the cells at one corner, at 264,000 leaves
+# so many that a sixteenth of them shows it
+@pytest.mark.parametrize("n,scale,power", [(3, 0.4, 1), (5, 1.0, 1), (9, 2.6, 1), (9, 5.0, 1),
+                                           (4, 1e6, 1), (9, 1.0, 4), (20, 1.0, 6), (20, 1.0, 1)])
+def test_grid_lists_of_every_length(cuda, n, scale, power):
     import torch
     from devil_ray_b200 import api, meshgen
     m = meshgen.trilinear_distorted_mesh(n, 2, 0.15, seed=11)
-    g = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda)
+    xyz = m.xyz if power == 1 else np.clip(m.xyz, 0, 1) ** np.float32(power)
+    g = api.UnstructuredMesh(m.ctrl_idx, xyz, m.order, device=cuda)
     b = g.get_bvh().build_grid(scale)
     torch.cuda.synchronize()
     dims, origin, inv = b.grid_geom
