@@ -136,14 +136,19 @@ class BVH:
         the same order; one 128-byte node per two binary levels)."""
         d = self.desc()
         dev = self.inner_nodes.device
-        ids = torch.empty(self.n_inner, dtype=torch.int32, device=dev)
-        if stream is not None:
-            ids.record_stream(stream)  # freed here, used there
+        # what is written on the stream comes from its own memory: a block of
+        # the current stream's may still be in use by work queued there
+        with torch.cuda.stream(stream):
+            ids = torch.empty(self.n_inner, dtype=torch.int32, device=dev)
         L.check(L.lib().drb_bvh_widen_plan(C.byref(d), _ptr(ids), _stream(stream)),
                 "drb_bvh_widen_plan")
-        self.wide_nodes = torch.empty((max(d.n_wide, 1), 32), dtype=torch.float32, device=dev)
-        L.check(L.lib().drb_bvh_widen_emit(C.byref(d), _ptr(ids), _ptr(self.wide_nodes),
-                                           d.n_wide, _stream(stream)), "drb_bvh_widen_emit")
+        with torch.cuda.stream(stream):
+            nodes = torch.empty((max(d.n_wide, 1), 32), dtype=torch.float32, device=dev)
+        if stream is not None:
+            nodes.record_stream(torch.cuda.current_stream(dev))  # locates run there
+        L.check(L.lib().drb_bvh_widen_emit(C.byref(d), _ptr(ids), _ptr(nodes), d.n_wide,
+                                           _stream(stream)), "drb_bvh_widen_emit")
+        self.wide_nodes = nodes
         self.n_wide, self.wide_depth = d.n_wide, d.wide_depth
         return self
 

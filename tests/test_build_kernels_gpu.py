@@ -271,6 +271,30 @@ def test_wide_plan_and_emit(cuda, kind, n_elem):
     assert np.array_equal(bits(b.wide_nodes.cpu().numpy()), bits(want))
 
 
+def test_widen_allocates_on_its_stream(cuda, monkeypatch):
+    """What widen(stream) writes on a stream is that stream's memory, not a
+    block that work queued on the current stream may still use."""
+    import torch
+    from devil_ray_b200 import api
+    b = _tree_mesh("scattered", 31, cuda).build_bvh()
+    want = b.widen().wide_nodes.cpu().numpy()
+    side = torch.cuda.Stream(cuda)
+    torch.cuda.synchronize()
+    empty, made_on = torch.empty, []
+
+    def recorded(*args, **kw):
+        made_on.append(torch.cuda.current_stream(cuda))
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", recorded)
+    b.widen(side)
+    monkeypatch.undo()
+    assert made_on and all(s == side for s in made_on)
+    assert torch.cuda.current_stream(cuda) != side
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(b.wide_nodes.cpu().numpy()), bits(want))
+
+
 # scales: lists of a few leaves, of some tens, of about a hundred (more than
 # 64 comparisons an entry: radix passes), and one cell with every leaf (more
 # than 64 leaves a cell: radix passes at once).  power: control points raised
