@@ -868,19 +868,18 @@ volume_kernel (VolumeParams vp, const Ray *__restrict__ rays, int n_rays, int *_
   }
 }
 
-// The plain march of few rays: a group of G lanes (4 to 32, a power of two)
-// takes G consecutive samples of one ray at once.  Every lane locates and
-// shades its own sample; then the group's samples are blended in ray order,
-// each lane repeating the same steps on values passed by shuffle, so the
-// result is the one-lane march's bit for bit (a plain sample does not depend
-// on the one before it, and the distances are the same repeated sums).
-// Samples behind the one that ends the ray are thrown away.  A group's round
-// takes several times a lane's sample, so a ray that ends within a few samples
-// loses by it: the rays come, in left, from volume_kernel's first part, which
-// keeps the rays whose samples are so opaque that they end soon.  Bound, like the
-// one-lane march, by the chains of node loads and Newton steps; the lanes give
-// the SMs enough of them.  256^2 pixels, 500 samples, 8^3 order-2 hexes: 4.38 ->
-// 1.99 ms a frame.
+// The plain march of few rays: a group of G lanes (8, 16 or 32) takes G
+// consecutive samples of one ray at once.  Every lane locates and shades its
+// own sample; then the group's samples are blended in ray order, each lane
+// repeating the same steps on values passed by shuffle, so the result is the
+// one-lane march's bit for bit (a plain sample does not depend on the one
+// before it, and the distances are the same repeated sums).  Samples behind the
+// one that ends the ray are thrown away.  A group's round takes several times a
+// lane's sample, so a ray that ends within a few samples loses by it: the rays
+// come, in left, from volume_kernel's first part, which keeps the rays whose
+// samples are so opaque that they end soon.  Bound, like the one-lane march, by
+// the chains of node loads and Newton steps; the lanes give the SMs enough of
+// them.  256^2 pixels, 500 samples, 8^3 order-2 hexes: 4.38 -> 1.99 ms a frame.
 template <int P, bool WIDE, int S>
 __global__ void __launch_bounds__ (128)
 volume_group_kernel (VolumeParams vp, int G, const RayMarch *__restrict__ left, int n_rays,
@@ -1086,19 +1085,19 @@ __global__ void fb_background_kernel (float4 *c, int n, float4 bg)
 // fill the SMs (512 threads each at 128 registers): its warps stay on
 // neighbouring rays at one depth, and no sample is thrown away.  With fewer
 // rays than half of that, the march is one chain of locates per lane and the
-// SMs idle, so a ray gets as many lanes as make about six waves of them, up to
-// 32.  Measured (us a frame, 1 lane / 8 / 16 / 32 lanes): 256^2 pixels, 500
-// samples, 8^3 order-2 hexes 4197 / 2217 / 2066 / 2358; 128^2, 300 samples,
-// 20^3 order 3 3163 / 1349 / 1078 / 998; 300^2, 200 samples, 10^3 x 6 order-2
-// tets 8629 / 7048 / 7005 / 7942; 512^2 of the order-3 hexes 6358 / 9177 / 9922
-// / 11461.  The coherent march keeps one lane: predicting several samples ahead
-// was up to twice as fast on small frames, but samples on shared faces then
-// fell to other elements than before.
+// SMs idle, so a ray gets 8 lanes, 16 (up to 3/8 of the SMs' lanes) or 32 (up to
+// 3/16): at most about six waves.  Measured (us a frame, 1 lane / 8 / 16 / 32
+// lanes): 256^2 pixels, 500 samples, 8^3 order-2 hexes 4197 / 2217 / 2066 /
+// 2358; 128^2, 300 samples, 20^3 order 3 3163 / 1349 / 1078 / 998; 300^2, 200
+// samples, 10^3 x 6 order-2 tets 8629 / 7048 / 7005 / 7942; 512^2 of the order-3
+// hexes 6358 / 9177 / 9922 / 11461.  The coherent march keeps one lane:
+// predicting several samples ahead was up to twice as fast on small frames, but
+// samples on shared faces then fell to other elements than before.
 int group_lanes (const VolumeParams &vp, int n)
 {
   const int lanes = 512 * sm_count ();
   if (vp.coherent || n > lanes / 2) return 1;
-  int G = 4;
+  int G = 8; // 6 * lanes / n is at least 12 here
   while (2 * G <= min (32, 6 * lanes / n)) G *= 2;
   return G;
 }
