@@ -37,7 +37,7 @@ constexpr int kOut = 3;
 // Inputs: the (P+1)^3 control points' 3 coordinates, then the point; K
 // padded to a multiple of 16 for the UMMA K steps.  Parameters, in one fp32
 // vector: W1 [128 x kIn], b1, W2 [128 x 128], b2, W3 [3 x 128], b3.  bf16
-// operand copies: W1 [128 x kInPad], W2, W2^T.
+// operand copies: W1 [128 x kInPad], W2 (the kernels read it both ways).
 template <int P> struct Net
 {
   static constexpr int kNd = (P + 1) * (P + 1) * (P + 1);
@@ -53,8 +53,7 @@ template <int P> struct Net
   static constexpr int kParams = kB3 + kOut;
   static constexpr int kBW1 = 0;
   static constexpr int kBW2 = kBW1 + kHid * kInPad;
-  static constexpr int kBW2T = kBW2 + kHid * kHid;
-  static constexpr int kBf16 = kBW2T + kHid * kHid;
+  static constexpr int kBf16 = kBW2 + kHid * kHid;
   // packed geometry rows: kCoords relative coordinates, then the origin
   static constexpr int kRowF4 = packed_stride (kNd, 3) / 4;
   // activation tile width: the layer-1 input, then the layer-2 input in
@@ -179,12 +178,7 @@ __global__ void prepare_kernel (const float *__restrict__ p, __nv_bfloat16 *__re
     const int r = t / N::kInPad, k = t - r * N::kInPad;
     wb[N::kBW1 + t] = __float2bfloat16_rn (k < N::kIn ? p[N::kW1 + r * N::kIn + k] : 0.f);
   }
-  if (t < kHid * kHid)
-  {
-    const int r = t / kHid, k = t - r * kHid;
-    wb[N::kBW2 + t] = __float2bfloat16_rn (p[N::kW2 + t]);
-    wb[N::kBW2T + t] = __float2bfloat16_rn (p[N::kW2 + k * kHid + r]);
-  }
+  if (t < kHid * kHid) wb[N::kBW2 + t] = __float2bfloat16_rn (p[N::kW2 + t]);
 }
 
 // ----------------------------------------------------------- features --

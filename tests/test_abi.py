@@ -123,3 +123,12 @@ def test_camera_moves_match_reference():
         got = np.array([*c.pos, *c.look_at], np.float32)
         assert np.array_equal(got.view(np.uint32), want[:6].view(np.uint32)), (got, want[:6])
         assert np.float32(c.fov) == np.float32(fov)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
+def test_guess_network_operands_are_the_two_layers(order):
+    """The bf16 operands are W1 and W2 and nothing else: the kernels read W2
+    both ways as it lies."""
+    from devil_ray_b200 import learned
+    lib = learned._lib()
+    assert lib.drb_mlp_bf16_count(order) == 128 * (lib.drb_mlp_input_width(order) + 128)
