@@ -523,7 +523,8 @@ __global__ void __launch_bounds__ (kNetThreads, 1) net_kernel (NetArgs a)
   if (!ok && tid == 0 && a.err) atomicExch (a.err, 1);
   if (TRAIN)
   {
-    // this CTA's sums to its slot (zeros where a wait ran out)
+    // this CTA's sums to its slot; where a wait ran out, zeros for the matrices and
+    // the finished tiles' sums for the rest (*err says that the step is void)
     float *out = a.partials + (size_t)blockIdx.x * partial_stride<P> ();
 #pragma unroll 1
     for (int c0 = 32 * g; c0 < kHid + kInPad; c0 += 32 * kNetGroups)
