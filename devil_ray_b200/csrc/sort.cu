@@ -3,21 +3,25 @@
 // the reference's LBVH build (linear_bvh_builder.cpp:120-135) and the RAJA
 // exclusive_scan of its compactions (array_utils.hpp:171-270).
 //
-// Sort pass (8-bit digit), bound by DRAM: 20 bytes per pair and pass.
+// Sort pass (8-bit digit): 20 bytes per pair, 0.34 ms of 30M pairs (1.8 TB/s), so
+// bound by the ranking's instructions rather than by the memory.
 //   hist_kernel     per-tile digit histogram in shared memory, written
 //                   digit-major
 //   digit_kernel    a block per digit scans its tiles' counts in place and
 //                   leaves the digit's total
-//   scatter_kernel  a tile of 4096 pairs per block.  Every warp ranks a
-//                   contiguous run of 512 pairs on its own (eight ballots a
-//                   row of 32 give the peers with the same digit, a
-//                   per-warp counter in shared memory the rank), so the
-//                   block synchronises only three times a tile; the pairs
+//   scatter_kernel  a tile of 4096 pairs (1024 of few) per block.  Every warp
+//                   ranks its eighth of them on its own (eight ballots a
+//                   row of 32 give the peers with the same digit, unless
+//                   the row is one run; a per-warp counter in shared
+//                   memory gives the rank), so the block synchronises
+//                   only three times a tile; the pairs
 //                   are then put in digit order in shared memory and leave
 //                   as runs of consecutive addresses.  Equal keys keep their
 //                   input order (stability), which makes the result
 //                   deterministic run to run.
-// Four passes over 8.65M pairs and three over 109M: 5.5 -> 4.0 ms.
+// Four passes over 8.65M pairs and three over 109M: 5.5 -> 4.0 ms.  30M random
+// keys of 30 bits 2.24 -> 1.34 ms, all of them equal 1.02 -> 1.21: runs as long as
+// a tile were coalesced without being put in order.
 #include "drb_common.cuh"
 #include "drb_internal.h"
 
@@ -28,28 +32,32 @@ namespace drb
 namespace
 {
 constexpr int kSortBlock = 256;
+// Keys per thread: 16, or 4 where tiles of 4096 would leave SMs without one: the
+// chain of a tile's rows is then what a pass waits for (30-bit keys, 16 / 4 a
+// thread: 100 of them 90 / 75 us, 10,000 106 / 80, 600,000 111 / 93).
 constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortBlock * kSortItems;
+constexpr int kSortItemsFew = 4;
 constexpr int kSortWarps = kSortBlock / kWarp;
 constexpr int kRadix = 256;
 static_assert (kRadix == kSortBlock, "a thread per digit");
 
+template <int ITEMS>
 __global__ void __launch_bounds__ (kSortBlock)
 hist_kernel (const unsigned *__restrict__ keys, int n, int shift, int ntiles, int *__restrict__ counts)
 {
   __shared__ int hist[kRadix];
   hist[threadIdx.x] = 0;
   __syncthreads ();
-  const long long base = (long long)blockIdx.x * kSortTile;
-  unsigned key[kSortItems];
+  const long long base = (long long)blockIdx.x * (kSortBlock * ITEMS);
+  unsigned key[ITEMS];
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
   {
     const long long idx = base + (long long)j * kSortBlock + threadIdx.x;
     key[j] = idx < n ? __ldg (keys + idx) : 0u;
   }
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
     if (base + (long long)j * kSortBlock + threadIdx.x < n) atomicAdd (&hist[(key[j] >> shift) & 0xffu], 1);
   __syncthreads ();
   counts[(size_t)threadIdx.x * ntiles + blockIdx.x] = hist[threadIdx.x];
@@ -122,44 +130,50 @@ digit_kernel (int *__restrict__ counts, int ntiles, int *__restrict__ totals)
 }
 
 // vals_in NULL: the values are the input positions.
+template <int ITEMS>
 __global__ void __launch_bounds__ (kSortBlock, 3)
 scatter_kernel (const unsigned *__restrict__ keys_in, const int *__restrict__ vals_in,
                 unsigned *__restrict__ keys_out, int *__restrict__ vals_out, int n, int shift,
                 int ntiles, const int *__restrict__ counts, const int *__restrict__ totals)
 {
-  __shared__ unsigned s_key[kSortTile];
-  __shared__ int s_val[kSortTile];
+  constexpr int kTile = kSortBlock * ITEMS;
+  __shared__ unsigned s_key[kTile];
+  __shared__ int s_val[kTile];
   __shared__ int wcnt[kSortWarps][kRadix];
   __shared__ int out_base[kRadix]; // digit's place in the output minus its place in the tile
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const long long base = (long long)blockIdx.x * kSortTile;
-  const int tile_n = (int)min ((long long)kSortTile, n - base);
-  unsigned key[kSortItems];
-  unsigned short rank[kSortItems];
+  const long long base = (long long)blockIdx.x * kTile;
+  const int tile_n = (int)min ((long long)kTile, n - base);
+  unsigned key[ITEMS];
+  unsigned short rank[ITEMS];
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
   {
-    const int i = warp * kWarp * kSortItems + j * kWarp + lane;
+    const int i = warp * kWarp * ITEMS + j * kWarp + lane;
     key[j] = i < tile_n ? __ldg (keys_in + base + i) : 0u;
   }
 #pragma unroll
   for (int q = 0; q < kRadix / kWarp; ++q) wcnt[warp][lane + q * kWarp] = 0;
   __syncwarp ();
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
   {
-    const bool valid = warp * kWarp * kSortItems + j * kWarp + lane < tile_n;
+    const bool valid = warp * kWarp * ITEMS + j * kWarp + lane < tile_n;
     const int digit = (key[j] >> shift) & 0xffu;
     unsigned peers = __ballot_sync (0xffffffffu, valid);
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
+    const int digit0 = __shfl_sync (0xffffffffu, digit, 0);
+    if (!__all_sync (0xffffffffu, digit == digit0)) // else the row is one run
     {
-      const bool set = (digit >> b) & 1;
-      const unsigned m = __ballot_sync (0xffffffffu, set);
-      peers &= set ? m : ~m;
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+      {
+        const bool set = (digit >> b) & 1;
+        const unsigned m = __ballot_sync (0xffffffffu, set);
+        peers &= set ? m : ~m;
+      }
     }
     int before = 0;
     if (valid) before = wcnt[warp][digit];
@@ -187,9 +201,9 @@ scatter_kernel (const unsigned *__restrict__ keys_in, const int *__restrict__ va
   }
   __syncthreads ();
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
   {
-    const int i = warp * kWarp * kSortItems + j * kWarp + lane;
+    const int i = warp * kWarp * ITEMS + j * kWarp + lane;
     if (i < tile_n)
     {
       const int at = wcnt[warp][(key[j] >> shift) & 0xffu] + rank[j];
@@ -199,7 +213,7 @@ scatter_kernel (const unsigned *__restrict__ keys_in, const int *__restrict__ va
   }
   __syncthreads ();
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
+  for (int j = 0; j < ITEMS; ++j)
   {
     const int i = j * kSortBlock + tid;
     if (i < tile_n)
@@ -352,11 +366,12 @@ int radix_sort_pairs (const unsigned *keys_in, const int *vals_in, unsigned *key
                       int *vals_out, int n, int bits, cudaStream_t s)
 {
   if (n <= 0) return DRB_OK;
-  const int ntiles = div_up (n, kSortTile);
+  const bool few = n < kSortBlock * kSortItems * sm_count ();
+  const int ntiles = div_up (n, kSortBlock * (few ? kSortItemsFew : kSortItems));
   const int passes = (bits + 7) / 8;
   Scratch scr (s);
-  int *counts = scr.alloc<int> ((size_t)kRadix * ntiles);
-  int *totals = scr.alloc<int> (kRadix);
+  int *counts = scr.alloc<int> ((size_t)kRadix * (ntiles + 1)); // and the digits' totals
+  int *totals = counts + (size_t)kRadix * ntiles;
   unsigned *kbuf = passes > 1 ? scr.alloc<unsigned> (n) : nullptr;
   int *vbuf = passes > 1 ? scr.alloc<int> (n) : nullptr;
   if (scr.err != cudaSuccess) return status_from (scr.err);
@@ -368,12 +383,18 @@ int radix_sort_pairs (const unsigned *keys_in, const int *vals_in, unsigned *key
     const bool to_out = ((passes - 1 - p) % 2) == 0;
     unsigned *kdst = to_out ? keys_out : kbuf;
     int *vdst = to_out ? vals_out : vbuf;
-    hist_kernel<<<ntiles, kSortBlock, 0, s>>> (ksrc, n, 8 * p, ntiles, counts);
+    if (few) hist_kernel<kSortItemsFew><<<ntiles, kSortBlock, 0, s>>> (ksrc, n, 8 * p, ntiles, counts);
+    else hist_kernel<kSortItems><<<ntiles, kSortBlock, 0, s>>> (ksrc, n, 8 * p, ntiles, counts);
     int st = check_launch ("hist_kernel");
     if (st) return st;
     digit_kernel<<<kRadix, min (1024, div_up (div_up (ntiles, 4), 32) * 32), 0, s>>> (counts, ntiles, totals);
     if ((st = check_launch ("digit_kernel"))) return st;
-    scatter_kernel<<<ntiles, kSortBlock, 0, s>>> (ksrc, vsrc, kdst, vdst, n, 8 * p, ntiles, counts, totals);
+    if (few)
+      scatter_kernel<kSortItemsFew><<<ntiles, kSortBlock, 0, s>>> (ksrc, vsrc, kdst, vdst, n, 8 * p, ntiles,
+                                                                   counts, totals);
+    else
+      scatter_kernel<kSortItems><<<ntiles, kSortBlock, 0, s>>> (ksrc, vsrc, kdst, vdst, n, 8 * p, ntiles,
+                                                                counts, totals);
     if ((st = check_launch ("scatter_kernel"))) return st;
     ksrc = kdst;
     vsrc = vdst;

@@ -110,7 +110,9 @@ def test_subboxes_match_restatement(cuda, dim, p, n):
 
 # ------------------------------------------------------- sort and scan --
 
-@pytest.mark.parametrize("n", [1, 31, 511, 4095, 4096, 4097, 3 * 4096 + 7, 300001])
+# tiles of 1024 keys below one tile of 4096 an SM, of 4096 above
+@pytest.mark.parametrize("n", [1, 31, 511, 1023, 1024, 1025, 4095, 4096, 4097, 3 * 4096 + 7, 300001,
+                               200 * 4096, 200 * 4096 + 1, 250 * 4096 - 5])
 @pytest.mark.parametrize("bits_", [1, 8, 9, 30, 32])
 def test_radix_sort_is_stable_at_tile_edges(cuda, n, bits_):
     import torch
