@@ -132,6 +132,7 @@ _SIGS = {
     "drb_framebuffer_composite_background": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p,
                                                        C.c_void_p]),
     "drb_kernel_launches": (C.c_ulonglong, []),
+    "drb_locate_small_queries": (C.c_int, []),
     "drb_locate_batched": (C.c_int, [C.POINTER(DrbMesh), C.POINTER(DrbBvh), C.c_void_p, C.c_int,
                                      C.POINTER(DrbNewtonOpts), C.c_void_p, C.c_void_p,
                                      C.c_void_p, DrbQueryStats, C.c_void_p]),

@@ -755,10 +755,8 @@ constexpr int kSmallPerSm = 700;
 constexpr int kSmallWarps = 16;
 constexpr int kSmallBlock = 64;
 
-bool small_batch (const drb_locate_config *cfg, int n)
-{
-  return !cfg && n <= kSmallPerSm * sm_count ();
-}
+int small_queries () { return kSmallPerSm * sm_count (); }
+bool small_batch (const drb_locate_config *cfg, int n) { return !cfg && n <= small_queries (); }
 
 LaunchShape small_batch_shape (int n)
 {
@@ -898,6 +896,8 @@ int locate_batched_ws (const drb_mesh *mesh, const drb_bvh *bvh, const float *pt
 } // namespace drb
 
 using namespace drb;
+
+extern "C" int drb_locate_small_queries (void) { return small_queries (); }
 
 extern "C" int drb_locate_batched (const drb_mesh *mesh, const drb_bvh *bvh, const float *pts,
                                    int n, const drb_newton_opts *opts,

@@ -303,13 +303,15 @@ class LearnedLocator:
         opts = L.DrbNewtonOpts(self.tol, self.max_steps, L.GUESS_GIVEN, guess.data_ptr())
         if bvh.grid_start is not None:
             # the points are in Morton order already: solve them in index order
+            # (few points without a configuration: one launch does that)
             cfg = L.DrbLocateConfig(128, 0, 64, 1, 0) if self.config is None else \
                 L.DrbLocateConfig(*(getattr(self.config, f) for f, _ in L.DrbLocateConfig._fields_))
             cfg.sort_queries = 0
+            few = self.config is None and n <= _lib().drb_locate_small_queries()
             bd = bvh.desc()
             L.check(_lib().drb_locate_batched(C.byref(self.mesh.desc()), C.byref(bd), _ptr(pts_s),
-                                              n, C.byref(opts), C.byref(cfg), _ptr(cell_s),
-                                              _ptr(ref_s), qs, _stream(stream)),
+                                              n, C.byref(opts), None if few else C.byref(cfg),
+                                              _ptr(cell_s), _ptr(ref_s), qs, _stream(stream)),
                     "drb_locate_batched")
         else:
             cfg = None if self.config is None else C.byref(self.config)

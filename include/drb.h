@@ -330,12 +330,16 @@ typedef struct drb_locate_config
  * warps popping chunks from a global atomic queue, idle lanes refilled by
  * ballot ranking, Newton solves of a warp run converged.  cfg NULL = the
  * library's choice: the default configuration { 128, 0, 64, 1, 0 }, or for a
- * small batch (up to 700 queries per SM) one launch without order or queue.  A
- * configuration that is given holds at every size.
+ * small batch (up to drb_locate_small_queries ()) one launch without order or
+ * queue.  A configuration that is given holds at every size.
  * Replaces UnstructuredMesh::locate (data_model/unstructured_mesh.cpp:124-148). */
 int drb_locate_batched (const drb_mesh *mesh, const drb_bvh *bvh, const float *pts, int n,
                         const drb_newton_opts *opts, const drb_locate_config *cfg, int *cell,
                         float *ref, drb_query_stats stats, void *stream);
+
+/* Largest batch that takes one launch when no configuration is given (700
+ * queries per SM of the current device). */
+int drb_locate_small_queries (void);
 
 /* drb_locate_batched without any device allocation, for callers that cannot
  * allocate when they locate points: a host application whose device memory

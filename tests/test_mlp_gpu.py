@@ -178,11 +178,13 @@ def test_hinted_locate_equals_plain_given_guess(cuda, setup):
     assert torch.equal(it0, it1) and torch.equal(ca0, ca1)
 
 
-def test_learned_locate_over_grid_equals_plain_given_guess(cuda, setup):
+@pytest.mark.parametrize("given", [False, True])
+def test_learned_locate_over_grid_equals_plain_given_guess(cuda, setup, given):
     """Over a BVH with grid lists the first candidates come from the query's
     cell and the solve runs through drb_locate_batched: the same first
     leaves as the tree walk, and the same cells, reference points,
-    iterations and candidates as drb_locate with those guesses."""
+    iterations and candidates as drb_locate with those guesses; in the one
+    launch of a small batch and with a given configuration."""
     import ctypes as C
     import torch
     from devil_ray_b200 import _lib as L
@@ -192,7 +194,8 @@ def test_learned_locate_over_grid_equals_plain_given_guess(cuda, setup):
     q = torch.as_tensor(meshgen.uniform_queries(50000, 23), device=cuda)
     tree = mesh.get_bvh()
     grid = tree.without_grid().build_grid(0.75)
-    ll = LG.LearnedLocator(mesh, model, tol=1e-5, max_steps=20, bvh=grid)
+    config = L.DrbLocateConfig(128, 0, 64, 1, 0) if given else None
+    ll = LG.LearnedLocator(mesh, model, tol=1e-5, max_steps=20, bvh=grid, config=config)
     order = ll._order.order(q)
     firsts = []
     for b in (tree, grid):
