@@ -415,7 +415,8 @@ class BatchedLocator:
     def capture(self, n: int) -> "LocateGraph":
         """A CUDA graph of this locator's batched locate over a static buffer
         of n queries (query order, persistent kernel and their scratch
-        allocations), for callers that locate many batches of one size."""
+        allocations, or a small batch's one launch), for callers that locate
+        many batches of one size."""
         return LocateGraph(self, n)
 
     def locate_host(self, host_points, out, chunk: int = 0, stream=None):
@@ -441,7 +442,8 @@ class LocateGraph:
     graph and replayed per batch: the queries go into `points` (or are
     passed to run()), results come back in `cell` / `ref`.  The graph holds
     the Morton ordering, the persistent kernel and their stream-ordered
-    scratch allocations, so a replay is one launch from the host."""
+    scratch allocations (a small batch's one launch without a configuration),
+    so a replay is one launch from the host."""
 
     def __init__(self, locator: BatchedLocator, n: int):
         dev = locator.mesh.device

@@ -3,8 +3,9 @@
 // the reference's LBVH build (linear_bvh_builder.cpp:120-135) and the RAJA
 // exclusive_scan of its compactions (array_utils.hpp:171-270).
 //
-// Sort pass (8-bit digit): 20 bytes per pair, 0.34 ms of 30M pairs (1.8 TB/s), so
-// bound by the ranking's instructions rather than by the memory.
+// Sort pass (8-bit digit): 20 bytes per pair, 0.34 ms of 30M pairs (1.8 TB/s):
+// bound by the latency of a tile's chain, three blocks an SM (36 % of the issue
+// slots, 12 % of DRAM at 8.65M pairs), not by the memory.
 //   hist_kernel     per-tile digit histogram in shared memory, written
 //                   digit-major
 //   digit_kernel    a block per digit scans its tiles' counts in place and

@@ -82,6 +82,35 @@ def test_few_rays_equal_many(cuda, kind, p, lit):
         assert torch.equal(parts[done], colors[done]) and torch.equal(seen[done], depths[done])
 
 
+# the partials of a few rays, in both parts of their march, against the same
+# rays among many
+@pytest.mark.parametrize("opacity", [0.02, 0.9, 1.0])
+def test_partials_of_few_rays_equal_many(cuda, opacity):
+    import torch
+    m, shape = _mesh("hex", 4, 2)
+    mesh = api.UnstructuredMesh(m.ctrl_idx, m.xyz, m.order, device=cuda, shape=shape)
+    values = torch.sin(9.0 * torch.as_tensor(m.xyz, device=cuda)).sum(1).float()
+    field = render.UnstructuredField(m.ctrl_idx, values, m.order, device=cuda, shape=shape)
+    c = meshgen.CAMERA
+    camera = render.Camera(512, 512, c["pos"], c["look_at"], c["up"], c["fov"])
+    vol = render.Volume(mesh, field)
+    table = render.ColorTable()
+    table.add_point(0.0, (0.1, 0.2, 0.9))
+    table.add_point(1.0, (0.9, 0.4, 0.1))
+    table.add_alpha(0.0, 0.0)
+    table.add_alpha(1.0, opacity)
+    vol.color_map().color_table(table)
+    vol.samples(60)
+    light = [render.PointLight.default(camera)]
+    rays = camera.create_rays(cuda)
+    some = rays[torch.arange(0, rays.shape[0], 37, device=cuda)].contiguous()
+    many, few = vol.integrate(rays, light), vol.integrate(some, light)
+    pixel = many[:, 0].contiguous().view(torch.int32)
+    kept = many[(pixel % 37 == 0).nonzero().squeeze(1)]
+    assert few.shape[0] > 500
+    assert torch.equal(few.view(torch.int32), kept.view(torch.int32))
+
+
 # a configuration that is given decides the launch at every size: with the
 # order there are launches before the locate kernel, with staged results one
 # behind it, without order or configuration there is one in all
