@@ -35,10 +35,14 @@ constexpr int kMaxDim = 4096;
 // The counting sort's lists are ordered by comparing every entry with its
 // list, so it is taken while an entry meets at most kOrderWork others on
 // average (on ordinary meshes about ten: 1.7 ms a 109M entries against 4.7 ms
-// of radix passes, whose time does not depend on the lists' length) and no list
-// keeps one warp busy for long (1024 entries: 32 rows of 1024 comparisons).
+// of radix passes, whose time does not depend on the lists' length) and while
+// the longest list does not keep its warp, whose 32 cells are neighbours and
+// likely as long, busy for longer than the passes would take: L^2 rounds of
+// about 2.2 ns against 34 ps an entry, L^2 * kOrderTail entries.  Graded 24^3
+// order-2 meshes (us a build, counting / passes): longest list 118 of 3.7M
+// entries 351 / 437, 251 of 2.1M 427 / 357, 854 of 3.7M 957 / 440.
 constexpr unsigned long long kOrderWork = 64;
-constexpr unsigned long long kOrderLongest = 1024;
+constexpr unsigned long long kOrderTail = 64;
 
 struct GridGeom
 {
@@ -151,12 +155,14 @@ DRB_D void table_range (const GridGeom &g, const float4 *__restrict__ table, int
 
 // Whether a graded mesh crowds its leaves into few cells: one warp of leaves
 // in kSampleWarps counts them into their first cells and raises *crowded when a
-// cell's count passes kOrderLongest.  Its list is then longer than that, so the
-// lists will take the radix passes whatever the counts are, and the counting is
-// left out: of 8.65M leaves, a quarter of them in one cell, it took 5 ms of a
-// build of 12.3, most of it atomics on that one counter and the few leaves that
-// cover thousands of cells each.  About 5 us where no cell is crowded.
+// cell gets more than kSampleCrowd, so that it holds about a thousand.  The
+// lists will then take the radix passes whatever the counts are, and the
+// counting is left out: of 8.65M leaves, a quarter of them in one cell, it took
+// 5 ms of a build of 12.3, most of it atomics on that one counter and the few
+// leaves that cover thousands of cells each.  About 5 us where no cell is
+// crowded.
 constexpr int kSampleWarps = 16;
+constexpr int kSampleCrowd = 64;
 
 __global__ void cell_sample_kernel (GridGeom g, const float4 *__restrict__ table, int n,
                                     int *__restrict__ counts, int *crowded)
@@ -167,7 +173,7 @@ __global__ void cell_sample_kernel (GridGeom g, const float4 *__restrict__ table
   int c0[3], c1[3];
   table_range (g, table, (int)k, c0, c1);
   const int cell = (c0[2] * g.dims[1] + c0[1]) * g.dims[0] + c0[0];
-  if (atomicAdd (counts + cell, 1) >= (int)kOrderLongest) *(volatile int *)crowded = 1;
+  if (atomicAdd (counts + cell, 1) >= kSampleCrowd) *(volatile int *)crowded = 1;
 }
 
 // Leaves per cell; with `sampled`, cell_sample_kernel has counted its leaves'
@@ -469,18 +475,18 @@ extern "C" int drb_bvh_grid_build (const drb_bvh *bvh, void *stream)
   box_table_kernel<<<div_up (bvh->n_inner, 256), 256, 0, s>>> (
       (const float4 *)bvh->inner_nodes, bvh->n_inner, bvh->leaf_nodes, table);
   if (int st = check_launch ("box_table_kernel")) return st;
-  // every leaf is in a list: with more than kOrderWork leaves a cell the lists
-  // are too long on average, and counting them would only crowd the atomics on
-  // a few counters
-  if (n > (long long)kOrderWork * n_cells) return sort_entries (bvh, g, n_cells, scr, s);
+  // with this many leaves a cell, each in two or more lists while cells are a
+  // few leaves wide, the lists are too long on average, and counting them would
+  // only crowd the atomics on a few counters
+  if (n > (long long)kOrderWork / 2 * n_cells) return sort_entries (bvh, g, n_cells, scr, s);
   int *counts = scr.alloc<int> (n_cells + 1);
   unsigned long long *stats = scr.alloc<unsigned long long> (4);
   if (!counts || !stats) return status_from (scr.err);
   int *crowded = reinterpret_cast<int *> (stats + 3);
   cudaMemsetAsync (counts, 0, sizeof (int) * (n_cells + 1), s);
   cudaMemsetAsync (stats, 0, 4 * sizeof (unsigned long long), s);
-  // (fewer leaves cannot raise the flag)
-  const bool sampled = n > (long long)kSampleWarps * (long long)kOrderLongest;
+  // (few leaves are counted in no time)
+  const bool sampled = n > 32768;
   if (sampled)
   {
     cell_sample_kernel<<<div_up (n, 256 * kSampleWarps), 256, 0, s>>> (g, table, n, counts, crowded);
@@ -500,7 +506,7 @@ extern "C" int drb_bvh_grid_build (const drb_bvh *bvh, void *stream)
   }
   if (h_stats[3]) return sort_entries (bvh, g, n_cells, scr, s);
   if (h_stats[0] >= (1ull << 31)) return too_many_entries ();
-  if (h_stats[1] > kOrderWork * h_stats[0] || h_stats[2] > kOrderLongest)
+  if (h_stats[1] > kOrderWork * h_stats[0] || h_stats[2] * h_stats[2] * kOrderTail > h_stats[0])
     return sort_entries (bvh, g, n_cells, scr, s);
   int *lists = scr.alloc<int> ((size_t)h_stats[0]);
   if (!lists) return status_from (scr.err);

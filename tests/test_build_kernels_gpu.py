@@ -299,11 +299,11 @@ def test_widen_allocates_on_its_stream(cuda, monkeypatch):
 
 # scales: lists of a few leaves, of some tens, of about a hundred (more than
 # 64 comparisons an entry: radix passes), and one cell with every leaf (more
-# than 64 leaves a cell: radix passes at once).  power: control points raised
+# than 32 leaves a cell: radix passes at once).  power: control points raised
 # to it, so that leaves crowd into the cells at one corner, at 264,000 leaves
 # so many that a sixteenth of them shows it
 @pytest.mark.parametrize("n,scale,power", [(3, 0.4, 1), (5, 1.0, 1), (9, 2.6, 1), (9, 5.0, 1),
-                                           (4, 1e6, 1), (9, 1.0, 4), (20, 1.0, 6), (20, 1.0, 1)])
+                                           (4, 1e6, 1), (9, 1.0, 4), (20, 1.0, 6), (20, 1.0, 1), (20, 1.5, 1.5)])
 def test_grid_lists_of_every_length(cuda, n, scale, power):
     import torch
     from devil_ray_b200 import api, meshgen
