@@ -475,9 +475,10 @@ __global__ void locate_persistent_kernel (DRB_PERSISTENT_ARGS)
 // Hexes with L1 rows, and every kind's grid scan at orders 1-2, held to the
 // registers that still give a full set of resident warps.  Left alone the
 // compiler's choice moves with small changes of the code: order 2 over grid
-// lists 89 registers (9 % slower than at 80, and 72 spills), order 3 109 to 115
-// (1M queries over the tree 414 us against 375 at 96, over grid lists 315
-// against 284); order 2 over the tree spills at 72 (545 us against 529).
+// lists 89 registers (9 % slower than at 80, and 72 spills), order 3 over grid
+// lists 108 (1M queries, 32^3 elements, linear guess: 354 us against 328 at 96)
+// and over the tree 92, scheduled worse than with 96 allowed (447 against 423);
+// order 2 over the tree 367 against 363 (and 72 spills: 545 against 529).
 template <int P> constexpr int max_regs () { return P == 3 ? 96 : 80; }
 template <int P, int MODE, int TRAV, int S = kTensor>
 __global__ void __maxnreg__ (max_regs<P> ()) locate_persistent_kernel_capped (DRB_PERSISTENT_ARGS)
